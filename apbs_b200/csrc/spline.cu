@@ -22,8 +22,8 @@
 // Forces: Vpmg_qfForce (vpmg.c:5862-5904 with qfForceSpline1 5906-6041,
 // qfForceSpline2 6043-6154 and qfForceSpline4 6156-6272), Vpmg_dbForce (5605-5860) and Vpmg_ibForce
 // (5440-5603) with Vacc_splineAccGradAtomNorm (src/generic/vacc.c:314-373).
-// One thread per atom walks the reference's loops in their order, so each
-// sum is taken in the reference's order.
+// One CTA per atom; its threads share the points of the reference's loops, so
+// each sum has the reference's terms in another (fixed) order.
 #include <algorithm>
 #include <vector>
 
@@ -298,6 +298,7 @@ __global__ void __launch_bounds__(kSplThreads) k_spline_fill(SplineArgs A) {
 // ---------------------------------------------------------------------------
 // forces
 // ---------------------------------------------------------------------------
+constexpr int kForceThreads = 128;
 struct ForceArgs {
   FillGeom G;
   int natoms;
@@ -431,9 +432,36 @@ __device__ __forceinline__ void surf_grad(const ForceArgs& A, int a, const doubl
   else spline_grad(center, A.win, infrad, apos, radius, grad);
 }
 
-__global__ void k_forces(ForceArgs A) {
-  const int a = blockIdx.x * blockDim.x + threadIdx.x;
-  if (a >= A.natoms) return;
+// Per-atom sums of the three components, added over the block's threads in a
+// fixed order (lanes, then warps); thread 0 has the result.
+__device__ __forceinline__ void force_sum(double v[3], double (*sh)[3]) {
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+#pragma unroll
+  for (int l = 0; l < 3; l++) {
+    v[l] = warp_sum(v[l]);
+    if (lane == 0) sh[wid][l] = v[l];
+  }
+  __syncthreads();
+  if (threadIdx.x == 0)
+#pragma unroll
+    for (int l = 0; l < 3; l++) {
+      double t = 0.0;
+      for (int w = 0; w < kForceThreads / 32; w++) t += sh[w][l];
+      v[l] = t;
+    }
+  __syncthreads();
+}
+
+// One CTA per atom, its threads striding over the grid points of each sum.
+// What bounds it is the FP64 arithmetic of the points near the surface (six
+// square roots and divisions each); with one thread per atom the kernel ran
+// for as long as one thread took over all its atom's points (13.8 ms for 700
+// atoms at 0.6 A, 0.15 ms now).  The sums are the reference's terms in
+// another order.
+__global__ void __launch_bounds__(kForceThreads) k_forces(ForceArgs A) {
+  __shared__ double sh[kForceThreads / 32][3];
+  const int a = blockIdx.x;
+  const int tid = threadIdx.x;
   const FillGeom& G = A.G;
   const int nx = G.g.nx, ny = G.g.ny, nz = G.g.nz;
   const double hx = G.h[0], hy = G.h[1], hzed = G.h[2];
@@ -444,7 +472,8 @@ __global__ void k_forces(ForceArgs A) {
   const double* u = A.u;
   auto IJK = [&](int i, int j, int k) { return ((size_t)k * ny + j) * nx + i; };
   double* out = A.out + 9 * (size_t)a;
-  for (int d = 0; d < 9; d++) out[d] = 0.0;
+  if (tid < 9) out[tid] = 0.0;
+  __syncthreads();
   int status = 1;
 
   // partition flag of Vpmg_setPart (vpmg.c:673-720) for the domain box
@@ -475,26 +504,29 @@ __global__ void k_forces(ForceArgs A) {
         const int jm2 = max((int)floor(jfloat) - 1, 0);
         const int kp2 = min((int)ceil(kfloat) + 1, nz - 1);
         const int km2 = max((int)floor(kfloat) - 1, 0);
-        for (int ii = im2; ii <= ip2; ii++) {
+        const int wj = jp2 - jm2 + 1, wk = kp2 - km2 + 1;
+        double t[3] = {0.0, 0.0, 0.0};
+        for (int c = tid; c < (ip2 - im2 + 1) * wj * wk; c += kForceThreads) {
+          const int ii = im2 + c / (wj * wk), jj = jm2 + (c / wk) % wj, kk = km2 + c % wk;
           const double mx = bspline2d(1.5 + ((double)ii - ifloat));
           const double dmx = dbspline2d(1.5 + ((double)ii - ifloat));
-          for (int jj = jm2; jj <= jp2; jj++) {
-            const double my = bspline2d(1.5 + ((double)jj - jfloat));
-            const double dmy = dbspline2d(1.5 + ((double)jj - jfloat));
-            for (int kk = km2; kk <= kp2; kk++) {
-              const double mz = bspline2d(1.5 + ((double)kk - kfloat));
-              const double dmz = dbspline2d(1.5 + ((double)kk - kfloat));
-              const double uv = u[IJK(ii, jj, kk)];
-              f[0] += (charge * dmx * my * mz * uv) / hx;
-              f[1] += (charge * mx * dmy * mz * uv) / hy;
-              f[2] += (charge * mx * my * dmz * uv) / hzed;
-            }
-          }
+          const double my = bspline2d(1.5 + ((double)jj - jfloat));
+          const double dmy = dbspline2d(1.5 + ((double)jj - jfloat));
+          const double mz = bspline2d(1.5 + ((double)kk - kfloat));
+          const double dmz = dbspline2d(1.5 + ((double)kk - kfloat));
+          const double uv = u[IJK(ii, jj, kk)];
+          t[0] += (charge * dmx * my * mz * uv) / hx;
+          t[1] += (charge * mx * dmy * mz * uv) / hy;
+          t[2] += (charge * mx * my * dmz * uv) / hzed;
         }
+        force_sum(t, sh);
+        if (tid == 0)
+          for (int l = 0; l < 3; l++) f[l] = t[l];
       }
     } else if (A.chgm == PMGB_CHGM_SPL4) {
       // handled below: qfForceSpline4 has no partition test
-    } else if (!((apos[0] <= xmin) || (apos[0] >= xmax) || (apos[1] <= ymin) ||
+    } else if (tid == 0 &&
+               !((apos[0] <= xmin) || (apos[0] >= xmax) || (apos[1] <= ymin) ||
                  (apos[1] >= ymax) || (apos[2] <= zmin) || (apos[2] >= zmax))) {
       // trilinear charges (qfForceSpline1)
       const double ifloat = (apos[0] - xmin) / hx;
@@ -548,27 +580,27 @@ __global__ void k_forces(ForceArgs A) {
     const int ip2 = min((int)ceil(ifloat) + 2, nx - 1), im2 = max((int)floor(ifloat) - 2, 0);
     const int jp2 = min((int)ceil(jfloat) + 2, ny - 1), jm2 = max((int)floor(jfloat) - 2, 0);
     const int kp2 = min((int)ceil(kfloat) + 2, nz - 1), km2 = max((int)floor(kfloat) - 2, 0);
+    const int wj = jp2 - jm2 + 1, wk = kp2 - km2 + 1;
     double e[3] = {0.0, 0.0, 0.0};
-    for (int ii = im2; ii <= ip2; ii++) {
+    for (int c = tid; c < (ip2 - im2 + 1) * wj * wk; c += kForceThreads) {
+      const int ii = im2 + c / (wj * wk), jj = jm2 + (c / wk) % wj, kk = km2 + c % wk;
       const double mi = (2.5 + ((double)(ii) - (ifloat)));
       const double mx = bspline4(mi), dmx = dbspline4(mi);
-      for (int jj = jm2; jj <= jp2; jj++) {
-        const double mj = (2.5 + ((double)(jj) - (jfloat)));
-        const double my = bspline4(mj), dmy = dbspline4(mj);
-        for (int kk = km2; kk <= kp2; kk++) {
-          const double mk = (2.5 + ((double)(kk) - (kfloat)));
-          const double mz = bspline4(mk), dmz = dbspline4(mk);
-          const double f = u[IJK(ii, jj, kk)];
-          e[0] += f * dmx * my * mz / hx;
-          e[1] += f * mx * dmy * mz / hy;
-          e[2] += f * mx * my * dmz / hzed;
-        }
-      }
+      const double mj = (2.5 + ((double)(jj) - (jfloat)));
+      const double my = bspline4(mj), dmy = dbspline4(mj);
+      const double mk = (2.5 + ((double)(kk) - (kfloat)));
+      const double mz = bspline4(mk), dmz = dbspline4(mk);
+      const double f = u[IJK(ii, jj, kk)];
+      e[0] += f * dmx * my * mz / hx;
+      e[1] += f * mx * dmy * mz / hy;
+      e[2] += f * mx * my * dmz / hzed;
     }
-    for (int d = 0; d < 3; d++) out[d] = e[d] * charge;
+    force_sum(e, sh);
+    if (tid == 0)
+      for (int d = 0; d < 3; d++) out[d] = e[d] * charge;
   }
   if (!A.boundary || part_id == 0.0) {
-    A.status[a] = status;
+    if (tid == 0) A.status[a] = status;
     return;
   }
 
@@ -590,50 +622,62 @@ __global__ void k_forces(ForceArgs A) {
         status = 0;  // "Atom off grid": the reference returns 0 here
       } else {
         double dbF[3] = {0.0, 0.0, 0.0};
-        for (int i = imin; i <= imax; i++) {
-          for (int j = jmin; j <= jmax; j++) {
-            for (int k = kmin; k <= kmax; k++) {
-              double gpos[3], dHx[3], dHy[3], dHz[3], dHxm[3], dHym[3], dHzm[3];
-              gpos[0] = (i + 0.5) * hx + xmin; gpos[1] = j * hy + ymin; gpos[2] = k * hzed + zmin;
-              const double Hxijk = (A.epsx[IJK(i, j, k)] - A.epsp) * depsi;
-              surf_grad(A, a, gpos, 0., apos, radius, dHx);
-              for (int l = 0; l < 3; l++) dHx[l] *= Hxijk;
-              gpos[0] = i * hx + xmin; gpos[1] = (j + 0.5) * hy + ymin; gpos[2] = k * hzed + zmin;
-              const double Hyijk = (A.epsy[IJK(i, j, k)] - A.epsp) * depsi;
-              surf_grad(A, a, gpos, 0., apos, radius, dHy);
-              for (int l = 0; l < 3; l++) dHy[l] *= Hyijk;
-              gpos[0] = i * hx + xmin; gpos[1] = j * hy + ymin; gpos[2] = (k + 0.5) * hzed + zmin;
-              const double Hzijk = (A.epsz[IJK(i, j, k)] - A.epsp) * depsi;
-              surf_grad(A, a, gpos, 0., apos, radius, dHz);
-              for (int l = 0; l < 3; l++) dHz[l] *= Hzijk;
-              gpos[0] = (i - 0.5) * hx + xmin; gpos[1] = j * hy + ymin; gpos[2] = k * hzed + zmin;
-              const double Hxim1jk = (A.epsx[IJK(i - 1, j, k)] - A.epsp) * depsi;
-              surf_grad(A, a, gpos, 0., apos, radius, dHxm);
-              for (int l = 0; l < 3; l++) dHxm[l] *= Hxim1jk;
-              gpos[0] = i * hx + xmin; gpos[1] = (j - 0.5) * hy + ymin; gpos[2] = k * hzed + zmin;
-              const double Hyijm1k = (A.epsy[IJK(i, j - 1, k)] - A.epsp) * depsi;
-              surf_grad(A, a, gpos, 0., apos, radius, dHym);
-              for (int l = 0; l < 3; l++) dHym[l] *= Hyijm1k;
-              gpos[0] = i * hx + xmin; gpos[1] = j * hy + ymin; gpos[2] = (k - 0.5) * hzed + zmin;
-              const double Hzijkm1 = (A.epsz[IJK(i, j, k - 1)] - A.epsp) * depsi;
-              surf_grad(A, a, gpos, 0., apos, radius, dHzm);
-              for (int l = 0; l < 3; l++) dHzm[l] *= Hzijkm1;
-              const double u0 = u[IJK(i, j, k)];
-              const double dbFmag = u0;
-              const double uxp = u[IJK(i + 1, j, k)], uxm = u[IJK(i - 1, j, k)];
-              const double uyp = u[IJK(i, j + 1, k)], uym = u[IJK(i, j - 1, k)];
-              const double uzp = u[IJK(i, j, k + 1)], uzm = u[IJK(i, j, k - 1)];
-              for (int l = 0; l < 3; l++) {
-                const double tg = (dHx[l] * (uxp - u0) + dHxm[l] * (uxm - u0)) / (hx * hx) +
-                                  (dHy[l] * (uyp - u0) + dHym[l] * (uym - u0)) / (hy * hy) +
-                                  (dHz[l] * (uzp - u0) + dHzm[l] * (uzm - u0)) / (hzed * hzed);
-                dbF[l] += (dbFmag * tg);
-              }
-            }
+        // every gradient is zero away from the shell |dist - radius| <= win;
+        // the six evaluation points lie half a spacing from the grid point
+        const double reach = A.win + 0.5 * fmax(hx, fmax(hy, hzed)) + 1.0e-6;
+        const double far2 = (radius + reach) * (radius + reach);
+        const double near2 = radius > reach ? (radius - reach) * (radius - reach) : -1.0;
+        const int wj = jmax - jmin + 1, wk = kmax - kmin + 1;
+        const int npts = (imax - imin + 1) * wj * wk;
+        for (int c = tid; c < npts; c += kForceThreads) {
+          const int i = imin + c % (imax - imin + 1);
+          const int j = jmin + (c / (imax - imin + 1)) % wj;
+          const int k = kmin + c / ((imax - imin + 1) * wj);
+          const double qx = i * hx - position[0], qy = j * hy - position[1],
+                       qz = k * hzed - position[2];
+          const double q2 = qx * qx + qy * qy + qz * qz;
+          if (q2 > far2 || q2 < near2) continue;
+          double gpos[3], dHx[3], dHy[3], dHz[3], dHxm[3], dHym[3], dHzm[3];
+          gpos[0] = (i + 0.5) * hx + xmin; gpos[1] = j * hy + ymin; gpos[2] = k * hzed + zmin;
+          const double Hxijk = (A.epsx[IJK(i, j, k)] - A.epsp) * depsi;
+          surf_grad(A, a, gpos, 0., apos, radius, dHx);
+          for (int l = 0; l < 3; l++) dHx[l] *= Hxijk;
+          gpos[0] = i * hx + xmin; gpos[1] = (j + 0.5) * hy + ymin; gpos[2] = k * hzed + zmin;
+          const double Hyijk = (A.epsy[IJK(i, j, k)] - A.epsp) * depsi;
+          surf_grad(A, a, gpos, 0., apos, radius, dHy);
+          for (int l = 0; l < 3; l++) dHy[l] *= Hyijk;
+          gpos[0] = i * hx + xmin; gpos[1] = j * hy + ymin; gpos[2] = (k + 0.5) * hzed + zmin;
+          const double Hzijk = (A.epsz[IJK(i, j, k)] - A.epsp) * depsi;
+          surf_grad(A, a, gpos, 0., apos, radius, dHz);
+          for (int l = 0; l < 3; l++) dHz[l] *= Hzijk;
+          gpos[0] = (i - 0.5) * hx + xmin; gpos[1] = j * hy + ymin; gpos[2] = k * hzed + zmin;
+          const double Hxim1jk = (A.epsx[IJK(i - 1, j, k)] - A.epsp) * depsi;
+          surf_grad(A, a, gpos, 0., apos, radius, dHxm);
+          for (int l = 0; l < 3; l++) dHxm[l] *= Hxim1jk;
+          gpos[0] = i * hx + xmin; gpos[1] = (j - 0.5) * hy + ymin; gpos[2] = k * hzed + zmin;
+          const double Hyijm1k = (A.epsy[IJK(i, j - 1, k)] - A.epsp) * depsi;
+          surf_grad(A, a, gpos, 0., apos, radius, dHym);
+          for (int l = 0; l < 3; l++) dHym[l] *= Hyijm1k;
+          gpos[0] = i * hx + xmin; gpos[1] = j * hy + ymin; gpos[2] = (k - 0.5) * hzed + zmin;
+          const double Hzijkm1 = (A.epsz[IJK(i, j, k - 1)] - A.epsp) * depsi;
+          surf_grad(A, a, gpos, 0., apos, radius, dHzm);
+          for (int l = 0; l < 3; l++) dHzm[l] *= Hzijkm1;
+          const double u0 = u[IJK(i, j, k)];
+          const double dbFmag = u0;
+          const double uxp = u[IJK(i + 1, j, k)], uxm = u[IJK(i - 1, j, k)];
+          const double uyp = u[IJK(i, j + 1, k)], uym = u[IJK(i, j - 1, k)];
+          const double uzp = u[IJK(i, j, k + 1)], uzm = u[IJK(i, j, k - 1)];
+          for (int l = 0; l < 3; l++) {
+            const double tg = (dHx[l] * (uxp - u0) + dHxm[l] * (uxm - u0)) / (hx * hx) +
+                              (dHy[l] * (uyp - u0) + dHym[l] * (uym - u0)) / (hy * hy) +
+                              (dHz[l] * (uzp - u0) + dHzm[l] * (uzm - u0)) / (hzed * hzed);
+            dbF[l] += (dbFmag * tg);
           }
         }
-        for (int l = 0; l < 3; l++)
-          out[3 + l] = -dbF[l] * hx * hy * hzed * deps * 0.5 * A.izmagic;
+        force_sum(dbF, sh);
+        if (tid == 0)
+          for (int l = 0; l < 3; l++)
+            out[3 + l] = -dbF[l] * hx * hy * hzed * deps * 0.5 * A.izmagic;
       }
     }
   }
@@ -646,48 +690,44 @@ __global__ void k_forces(ForceArgs A) {
     const double rtot = (A.irad + radius + A.win);
     const double rtot2 = rtot * rtot;
     double ibF[3] = {0.0, 0.0, 0.0};
-    const double ddx = rtot + 0.5 * hx;
+    // the points within rtot of the atom (the reference's nested ranges hold
+    // every point that passes its distance test)
+    const double ddx = rtot + 0.5 * hx, ddy = rtot + 0.5 * hy, ddz = rtot + 0.5 * hzed;
     const int imin = max(0, (int)ceil((position[0] - ddx) / hx));
     const int imax = min(nx - 1, (int)floor((position[0] + ddx) / hx));
-    for (int i = imin; i <= imax; i++) {
+    const int jmin = max(0, (int)ceil((position[1] - ddy) / hy));
+    const int jmax = min(ny - 1, (int)floor((position[1] + ddy) / hy));
+    const int kmin = max(0, (int)ceil((position[2] - ddz) / hzed));
+    const int kmax = min(nz - 1, (int)floor((position[2] + ddz) / hzed));
+    const int wi = imax - imin + 1, wj = jmax - jmin + 1;
+    const int npts = wi > 0 && wj > 0 ? wi * wj * max(0, kmax - kmin + 1) : 0;
+    for (int c = tid; c < npts; c += kForceThreads) {
+      const int i = imin + c % wi, j = jmin + (c / wi) % wj, k = kmin + c / (wi * wj);
       const double dx2 = (position[0] - hx * i) * (position[0] - hx * i);
-      double dy;
-      if (rtot2 > dx2) dy = sqrt(rtot2 - dx2) + 0.5 * hy;
-      else dy = 0.5 * hy;
-      const int jmin = max(0, (int)ceil((position[1] - dy) / hy));
-      const int jmax = min(ny - 1, (int)floor((position[1] + dy) / hy));
-      for (int j = jmin; j <= jmax; j++) {
-        const double dy2 = (position[1] - hy * j) * (position[1] - hy * j);
-        double dz;
-        if (rtot2 > (dx2 + dy2)) dz = sqrt(rtot2 - dx2 - dy2) + 0.5 * hzed;
-        else dz = 0.5 * hzed;
-        const int kmin = max(0, (int)ceil((position[2] - dz) / hzed));
-        const int kmax = min(nz - 1, (int)floor((position[2] + dz) / hzed));
-        for (int k = kmin; k <= kmax; k++) {
-          const double dz2 = (k * hzed - position[2]) * (k * hzed - position[2]);
-          if ((dz2 + dy2 + dx2) <= rtot2) {
-            double gpos[3], tgrad[3];
-            gpos[0] = i * hx + xmin;
-            gpos[1] = j * hy + ymin;
-            gpos[2] = k * hzed + zmin;
-            surf_grad(A, a, gpos, A.irad, apos, radius, tgrad);
-            const double uv = u[IJK(i, j, k)], kv = A.kappa[IJK(i, j, k)];
-            double fmag;
-            if (A.nonlin) {
-              fmag = 0.0;
-              for (int m = 0; m < A.nion; m++)
-                fmag += kv * A.ion_conc[m] * (cap_exp(-A.ion_q[m] * uv) - 1.0) / A.ionstr;
-            } else {
-              fmag = (uv * uv) * kv;
-            }
-            for (int l = 0; l < 3; l++) ibF[l] += (A.zkappa2 * fmag * tgrad[l]);
-          }
-        }
+      const double dy2 = (position[1] - hy * j) * (position[1] - hy * j);
+      const double dz2 = (k * hzed - position[2]) * (k * hzed - position[2]);
+      if (!((dz2 + dy2 + dx2) <= rtot2)) continue;
+      double gpos[3], tgrad[3];
+      gpos[0] = i * hx + xmin;
+      gpos[1] = j * hy + ymin;
+      gpos[2] = k * hzed + zmin;
+      surf_grad(A, a, gpos, A.irad, apos, radius, tgrad);
+      const double uv = u[IJK(i, j, k)], kv = A.kappa[IJK(i, j, k)];
+      double fmag;
+      if (A.nonlin) {
+        fmag = 0.0;
+        for (int m = 0; m < A.nion; m++)
+          fmag += kv * A.ion_conc[m] * (cap_exp(-A.ion_q[m] * uv) - 1.0) / A.ionstr;
+      } else {
+        fmag = (uv * uv) * kv;
       }
+      for (int l = 0; l < 3; l++) ibF[l] += (A.zkappa2 * fmag * tgrad[l]);
     }
-    for (int l = 0; l < 3; l++) out[6 + l] = ibF[l] * 0.5 * hx * hy * hzed * A.izmagic;
+    force_sum(ibF, sh);
+    if (tid == 0)
+      for (int l = 0; l < 3; l++) out[6 + l] = ibF[l] * 0.5 * hx * hy * hzed * A.izmagic;
   }
-  A.status[a] = status;
+  if (tid == 0) A.status[a] = status;
 }
 
 }  // namespace
@@ -818,7 +858,7 @@ extern "C" int pmgb_forces(pmgb_solver* s, double* qf, double* db, double* ib) {
   }
   A.out = s->d_forces;
   A.status = reinterpret_cast<int*>(s->d_forces + 9 * (size_t)natoms);
-  k_forces<<<(natoms + 127) / 128, 128, 0, st>>>(A);
+  k_forces<<<natoms, kForceThreads, 0, st>>>(A);
   note_launches(1);
   std::vector<double> h(9 * (size_t)natoms);
   std::vector<int> stat(natoms);
