@@ -7,6 +7,9 @@
 // global sums (norms, dot products) are reassociated (tree reductions).
 #include <cooperative_groups.h>
 
+#include <algorithm>
+#include <type_traits>
+
 #include "gs7_rb.cuh"
 #include "mg_kernels.cuh"
 
@@ -887,42 +890,95 @@ int launch_gs27_planes(cudaStream_t s, Grid g, Op op, const double* cc, const do
 }
 
 // ---------------------------------------------------------------------------
-// The same schedule, one CTA per interior plane, with the CTA's plane and its
-// two neighbour planes held in shared memory and every update passed to the
-// neighbour planes through a mailbox in global memory instead of by step
-// counters.
+// The same order with one CTA per interior plane and every update passed to
+// the neighbour planes by value instead of by step counters: into the
+// neighbour's shared memory where it belongs to the same cluster, through a
+// mailbox in global memory where it does not.
 //
-// The GS update of point (i, j, k) in half-sweep q goes into the CTA's own
-// copy and into mailbox slot (k, q, j, m) as two 64-bit words, each holding
-// one 32-bit half of the value beside the launch's tag.  A reader polls the
-// slot until both tags are the launch's: the value validates itself, so no
-// fence and no counter lies between one plane's update and the neighbour's
-// use of it.  Every slot is written once per launch, so nothing is
-// overwritten before it is read, and the tags of earlier launches never
-// match.
+// The GS update of point (i, j, k) in half-sweep q travels as two 64-bit
+// words, each holding one 32-bit half of the value beside a tag.  A reader
+// polls the slot until both tags are the ones it expects: the value validates
+// itself, so no fence and no counter lies between one plane's update and the
+// neighbour's use of it.  A global slot (k, q, j, m) is written once per
+// launch and tagged with the launch count of its plane.  The slots in shared
+// memory (the inbox) are a ring over the rows, tagged with the launch and the
+// lap; a neighbour is never more than wlag rows ahead of its reader (below),
+// and the ring holds wlag + 2.
 //
-// A CTA copies a neighbour's updates into its copy of that plane at the step
-// that first needs them: half-sweep q at row j takes row j+1 of the lower
-// plane's half-sweep q (finished one wavefront earlier) and row j+1 of the
-// upper plane's half-sweep q-1 (finished wlag-3 wavefronts earlier), and at
-// j = 1 row 1 of both too.  The rows a step reads then hold exactly the
-// values the sequential order reads (the lower plane swept by this
-// half-sweep, the upper one by the earlier ones), and the rows a step
-// changes lie at least two rows from those any other half-sweep reads in
-// that step or the one before, so one block barrier per step orders
-// everything.  The iterates are bitwise those of k_gs27_wave whatever the
-// order in which the planes run; tests/test_gs27_wave_deps.py runs this rule
-// on adversarial interleavings.
+// Each half-sweep q of a plane has its own warps, which go through its rows in
+// steps.  Step j first takes mail into the CTA's copies of the neighbour planes
+// -- row j+1 of the lower plane's half-sweep q, and for the next step row j+2 of
+// the upper plane's half-sweep q-1 -- then updates row j.  A half-sweep follows
+// the one before it on its plane by at least three rows and at most wlag.  The
+// rows an update reads hold exactly the values the sequential order reads (the
+// lower plane swept by this half-sweep, the upper one by the earlier ones), and
+// the rows a step changes lie outside those any other half-sweep may still
+// read.  The iterates are bitwise those of k_gs27_wave whatever the order in
+// which planes and half-sweeps run; tests/test_gs27_mail_ring.py runs this rule
+// on adversarial interleavings, and how far a neighbour gets ahead.
+//
+// What bounds it: the wave reaches plane k two steps and one hand-over after
+// plane k-1, so its length is (planes) x (step + hand-over) + (rows) x step.
+// A hand-over through global memory costs an L2 write and at least one polling
+// round trip, about as much as the rest of a step; a store to a neighbour SM's
+// shared memory and a poll of the own one cost a fraction of it.  The rest of
+// the step is kept short:
+//  * Only three of the 26 neighbours change in the step before an update (the
+//    lower plane's (i, j+1) and the own plane's (i+-1, j-1)).  The other 23
+//    products, and the sums that precede them in the reference's order, are
+//    made at the end of the previous step, after its updates were sent.
+//  * Coefficients in the order an update reads them (k_gs27_pack): per row and
+//    colour, 14 pairs of doubles for each point, contiguous over the points of
+//    the colour -- the 26 couplings, the diagonal D = oC + cc and 1/D.  Read
+//    from the 14 operator arrays a colour uses half of each sector and 28
+//    address computations per point.  A warp of its own brings them in by bulk
+//    copies, which take no part of the load pipe the workers' critical loads
+//    wait for.
+//  * A ring of rows of the three planes instead of whole planes (nx up to 113
+//    instead of 97), loaded by the same warp.
+//  * Half-sweeps are not in lockstep: one's waits overlap another's products.
+//  * The last two half-sweeps store their updates to x themselves, so nothing
+//    follows the last step; an iterate known to be zero is neither written nor
+//    loaded.
+//  * A quotient by the prefetched reciprocal, correctly rounded (div_by).
+//  * At the edge of a cluster, couriers (four warps) poll the foreign
+//    neighbour's global slots, two rows at a time, and put the values into the
+//    inbox: the polls' round trips are off the workers' path.
+//  * The residual is a kernel of its own: it would double the loads of a step
+//    for a pass that needs no order.
+// Measured (two sweeps and the residual, lag 6; in brackets the kernels before,
+// whole planes in shared memory and a global mailbox, at 113^3 step counters):
+// 17^3 49 us (66), 33^3 96 (126), 49^3 150 (203), 65^3 212 (289), 81^3 300 (455),
+// 97^3 460 (744), 113^3 558 (1244).
+//
+// Why a neighbour stays within wlag rows: half-sweep q of the lower plane can
+// run row J only after this plane's half-sweep q-1 ran row J+1, which is at
+// most wlag rows ahead of this plane's half-sweep q (half-sweep 0 is held by
+// the lower plane's own half-sweep 1 in the same way); and the upper plane's
+// half-sweep q-1 can run row J only after this plane's ran J+1.  For the same
+// reason x may be stored and loaded in place: when half-sweep q >= 1 of a plane
+// updates row j, both neighbours' first half-sweeps have passed it and loaded
+// it.
 //
 // The counters hold the launch count of each plane (the tag is that plus
-// one); a CTA writes its plane back to x at the end, after both neighbours
-// have read theirs (with two or more half-sweeps a CTA waits on both
-// neighbours' updates before it finishes).  A wait that runs out is counted
-// in *err like the counter kernel's.
+// one).  A wait that runs out is counted in *err like the counter kernel's.
 // ---------------------------------------------------------------------------
-constexpr int kMailThreads = 384;
-constexpr int kMailPoll = 2;     // mailbox slots one thread polls per step, at most
-constexpr int kMailHalfMax = 4;  // half-sweeps per launch the mailbox holds
+constexpr int kMailWorkers = 256;   // at most: four half-sweeps of two warps
+constexpr int kMailCouriers = 96;   // and one warp that loads
+constexpr int kMailHelpers = kMailCouriers + 32;
+constexpr int kMailHalfMax = 4;     // half-sweeps per launch
+constexpr int kMailLagMax = 6;      // rows between successive half-sweeps, at most
+// rows of x a CTA keeps of each plane: from the last half-sweep's lowest to
+// the first one's highest, and some loaded ahead
+constexpr int kMailRows = 26;
+constexpr int kMailInRows = 8;      // rows of the inbox
+static_assert(kMailRows >= kMailLagMax * (kMailHalfMax - 1) + 5 &&
+              kMailInRows >= kMailLagMax + 2, "rings of k_gs27_mail");
+constexpr int kMailPutMax = 2 * kMailHalfMax - 1;  // half-sweeps the inbox holds: 4 of the lower
+                                                   // plane, 3 of the upper
+constexpr int kPackPairs = 14;      // pairs of doubles per point of k_gs27_pack
+// stages of packed coefficients per half-sweep, as shared memory allows
+__host__ __device__ constexpr int mail_stages(int hp) { return hp <= 40 ? 3 : 2; }
 
 __device__ __forceinline__ void mail_put(unsigned long long* p, double v, unsigned tag) {
   const unsigned long long b = (unsigned long long)__double_as_longlong(v);
@@ -935,269 +991,590 @@ __device__ __forceinline__ void mail_load(const unsigned long long* p, unsigned 
                                           unsigned long long& w1) {
   asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(w0), "=l"(w1) : "l"(p));
 }
+// a / b with y = RN(1/b): P. Markstein's quotient (IBM J. Res. Dev. 34, 1990):
+// with y correctly rounded, a quotient within one ulp of a / b is corrected
+// to the rounded one by its exact remainder times y; the first correction
+// brings a*y (up to 1.5 ulp off) there.  Outside the range where a remainder
+// could underflow or overflow, the division itself.
+__device__ __forceinline__ double div_by(double a, double b, double y) {
+  const double q0 = a * y;
+  const double q1 = __fma_rn(__fma_rn(-b, q0, a), y, q0);
+  const double q2 = __fma_rn(__fma_rn(-b, q1, a), y, q1);
+  const unsigned e = (unsigned)__double2hiint(q0) & 0x7fffffffu;  // exponent of the quotient
+  if (e - 0x10000000u < 0x60000000u || a == 0.0) return q2;       // 2^-767 .. 2^769, or 0 / b
+  return a / b;
+}
+
+static int mail_hr(Grid g) { return (g.nx - 1) / 2; }         // points of one colour in a row
+static int pack_hr(Grid g) { return (mail_hr(g) + 7) & ~7; }  // the same, in whole lines
 
 size_t mail_words(Grid g) {
-  const size_t hr = (g.nx - 1) / 2;
-  return 2 * (size_t)(g.nz - 2) * kMailHalfMax * (g.ny - 2) * hr;
+  return 2 * (size_t)(g.nz - 2) * kMailHalfMax * (g.ny - 2) * mail_hr(g);
 }
-// shared memory of k_gs27_mail: three planes, each row split by the parity
-// of i into two runs of (nx + 1) / 2 values
+size_t gs27_pack_doubles(Grid g) {
+  return (size_t)(g.nz - 2) * (g.ny - 2) * 2 * kPackPairs * 2 * pack_hr(g);
+}
 static size_t mail_smem(Grid g) {
-  return 3 * (size_t)2 * ((g.nx + 1) / 2) * g.ny * sizeof(double);
+  const size_t hp = pack_hr(g);
+  return mail_stages((int)hp) * kMailHalfMax * kPackPairs * hp * 16 +
+         3 * kMailRows * 2 * (hp + 2) * sizeof(double) + kMailPutMax * kMailInRows * hp * 16;
 }
 
-__global__ void __launch_bounds__(kMailThreads, 1)
-    k_gs27_mail(Grid g, Op op, const double* __restrict__ cc, const double* __restrict__ fc,
-                double* x, double* r, int nhalf, int first_parity, int do_resid,
-                unsigned* counters, int* err, int wlag, unsigned long long* mail) {
-  // planes k-1, k, k+1 of x; each row as its even-i values then its odd-i
-  // values, so the points one warp updates (one colour of a row) and each of
-  // their stencil neighbours lie contiguously: two shared-memory wavefronts
-  // per warp load instead of four
-  extern __shared__ double pl[];
-  const int nx = g.nx, ny = g.ny, nz = g.nz;
-  const int pn = nx * ny;
-  const int H = (nx + 1) / 2;
-  const int ps = 2 * H * ny;  // doubles per plane in shared memory
-  auto sidx = [&](int i, int j) -> int { return (2 * j + (i & 1)) * H + (i >> 1); };
-  const size_t sy = nx, sz = (size_t)pn;
-  const int tmin = 1 + 2 * 1, tmax = (ny - 2) + 2 * (nz - 2);
-  const int nphase = nhalf + (do_resid ? 1 : 0);
-  const int resid_lag = wlag * nhalf;
-  const int last_start = do_resid ? resid_lag : wlag * (nhalf - 1);
-  const int nsteps = (tmax - tmin + 1) + last_start;
+// The packed coefficients of a 27-point level; coef 0: only the pair (D, 1/D),
+// for another Helmholtz term cc on the same operator.
+__global__ void k_gs27_pack(Grid g, Op op, const double* __restrict__ cc, double2* pk, int hp,
+                            int coef) {
+  const int nx = g.nx, ny = g.ny;
+  const int hr = (nx - 1) / 2;
+  const size_t sy = nx, sz = (size_t)nx * ny;
+  const size_t n = (size_t)(g.nz - 2) * (ny - 2) * 2 * hp;
+  for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n;
+       e += (size_t)gridDim.x * blockDim.x) {
+    int m, par, row;
+    split3(e, hp, 2, m, par, row);
+    const int j = 1 + row % (ny - 2), k = 1 + row / (ny - 2);
+    const int i = 1 + (((1 + j + k) & 1) != par) + 2 * m;
+    double2* out = pk + (e / hp) * (size_t)kPackPairs * hp + m;
+    if (m >= hr || i > nx - 2) {
+      if (coef)
+        for (int t = 0; t < kPackPairs; t++) out[(size_t)t * hp] = make_double2(0.0, 0.0);
+      continue;
+    }
+    const size_t id = g.idx(i, j, k);
+    const double d = op.c[OC][id] + cc[id];
+    out[(size_t)13 * hp] = make_double2(d, 1.0 / d);
+    if (!coef) continue;
+    Coef27 C;
+    load_coef27(op, cc, cc, id, sy, sz, C);
+    double v[26];
+#pragma unroll
+    for (int t = 0; t < 8; t++) v[t] = C.o[t];
+#pragma unroll
+    for (int t = 0; t < 9; t++) {
+      v[8 + t] = C.u[t];
+      v[17 + t] = C.d[t];
+    }
+#pragma unroll
+    for (int t = 0; t < 13; t++) out[(size_t)t * hp] = make_double2(v[2 * t], v[2 * t + 1]);
+  }
+}
+
+void launch_gs27_pack(cudaStream_t s, Grid g, Op op, const double* cc, double* pk, int coef) {
+  const int hp = pack_hr(g);
+  const size_t n = (size_t)(g.nz - 2) * (g.ny - 2) * 2 * hp;
+  k_gs27_pack<<<blocks_for(n, 128), 128, 0, s>>>(g, op, cc, reinterpret_cast<double2*>(pk), hp,
+                                                 coef);
+}
+
+// What one step leaves for the next step's update of a point: the sums and
+// products that do not wait for that step's mail.
+struct Ready27 {
+  double o, u, d0, d2, d3, d4, d5, d6, d7, d8;  // partial tO, tU, products of tD
+  double a1, a6, a7;                            // couplings of the late neighbours
+  double f, diag, rdiag;
+};
+
+// a cluster's shared memory: the address of this CTA's `p` in CTA `rank`
+__device__ __forceinline__ unsigned cluster_addr(const void* p, int rank) {
+  unsigned a = (unsigned)__cvta_generic_to_shared(p), r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ void inbox_put(unsigned addr, unsigned long long w0,
+                                          unsigned long long w1) {
+  asm volatile("st.relaxed.cluster.shared::cluster.v2.u64 [%0], {%1, %2};" ::"r"(addr), "l"(w0),
+               "l"(w1)
+               : "memory");
+}
+__device__ __forceinline__ void inbox_load(unsigned addr, unsigned long long& w0,
+                                           unsigned long long& w1) {
+  asm volatile("ld.relaxed.cluster.shared::cluster.v2.u64 {%0, %1}, [%2];"
+               : "=l"(w0), "=l"(w1)
+               : "r"(addr)
+               : "memory");
+}
+__device__ __forceinline__ bool mail_is(unsigned long long w0, unsigned long long w1,
+                                        unsigned tag) {
+  return (unsigned)(w0 >> 32) == tag && (unsigned)(w1 >> 32) == tag;
+}
+
+__device__ __forceinline__ bool mbar_done(unsigned bar, unsigned parity) {
+  unsigned ok;
+  asm volatile(
+      "{\n .reg .pred p;\n mbarrier.test_wait.parity.acquire.cta.shared::cta.b64 p, [%1], %2;\n"
+      " selp.u32 %0, 1, 0, p;\n}"
+      : "=r"(ok)
+      : "r"(bar), "r"(parity)
+      : "memory");
+  return ok != 0u;
+}
+
+// HP: pack_hr of the level.  A single warp per scheduler runs most of a step,
+// so its length is its instruction count: strides are compile-time constants,
+// rows and slots are reached by increments, and the two colour offsets of a
+// row have a copy of the step each (a thread alternates between them).
+template <int HP>
+__global__ void __launch_bounds__(kMailWorkers + kMailHelpers, 1)
+    k_gs27_mail(Grid g, const double2* __restrict__ pk, const double* __restrict__ fc, double* x,
+                int x_zero, int nhalf, int first_parity, unsigned* counters, int* err, int wlag,
+                unsigned long long* mail) {
+  constexpr unsigned RUN = HP + 2;              // values of one column parity of a row (even)
+  constexpr unsigned RL = 2 * RUN;              // a row: its even-i values, then its odd-i ones
+  constexpr unsigned PS = RL * kMailRows;       // a plane
+  constexpr unsigned IROW = 2 * HP;             // words of an inbox row
+  constexpr unsigned IBOX = IROW * kMailInRows; // words of one half-sweep's inbox
+  constexpr int NS = mail_stages(HP);
+  constexpr unsigned REC = kPackPairs * HP;     // pairs of one row and colour
+  // stages of coefficients [half-sweep][stage], planes k-1, k, k+1 of x, the
+  // inbox (half-sweeps 0-3 of the lower plane, 0-2 of the upper)
+  extern __shared__ __align__(128) double2 coef[];
+  double* ring = reinterpret_cast<double*>(coef + kMailHalfMax * NS * REC);
+  unsigned long long* inbox = reinterpret_cast<unsigned long long*>(ring + 3 * PS);
+  __shared__ unsigned long long full[kMailHalfMax][NS];
+  __shared__ unsigned tag_sh;
+  // the last row of x loaded; per half-sweep the step all its threads have
+  // entered (row before it updated, products of its row made)
+  __shared__ volatile int rows_sh, prog_sh[kMailHalfMax];
+  __shared__ volatile int failed_sh;
+  cg::cluster_group cl = cg::this_cluster();
+  const int rank = (int)cl.block_rank(), clsize = (int)cl.num_blocks();
+  const int nx = g.nx, ny = g.ny;
   const int hr = (nx - 1) / 2;
   const int c = blockIdx.x, k = 1 + c;
-  const int ncta = gridDim.x;
-  double* P0 = pl;
-  double* P1 = pl + ps;
-  double* P2 = pl + 2 * ps;
-  __shared__ unsigned tag_sh;
-  __shared__ volatile int failed_sh;
+  const int ncta = g.nz - 2;  // CTAs beyond the last plane only meet the cluster's barriers
+  const int nwork = blockDim.x - kMailHelpers;
+  const bool has_plane = c < ncta;
   if (threadIdx.x == 0) {
-    tag_sh = counters[c] + 1u;
+    tag_sh = has_plane ? counters[c] + 1u : 0u;
+    rows_sh = 3;
     failed_sh = 0;
+    for (int q = 0; q < kMailHalfMax; q++) prog_sh[q] = -2;
+    for (int q = 0; q < kMailHalfMax; q++)
+      for (int t = 0; t < NS; t++)
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(
+                         (unsigned)__cvta_generic_to_shared(&full[q][t]))
+                     : "memory");
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  {
-    // the three planes are contiguous in x; asynchronous 8-byte copies keep
-    // all of them in flight at once
-    const double* src = x + (size_t)(k - 1) * pn;
-    for (int e = threadIdx.x; e < 3 * pn; e += blockDim.x) {
-      const int p3 = e / pn, e2 = e - p3 * pn;
-      const int jj = e2 / nx, ii = e2 - jj * nx;
-      const unsigned dst = (unsigned)__cvta_generic_to_shared(pl + p3 * ps + sidx(ii, jj));
-      asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(src + e)
-                   : "memory");
+  // no tag is 0
+  for (unsigned e = threadIdx.x; e < kMailPutMax * IBOX; e += blockDim.x) inbox[e] = 0ull;
+  // row `row` of the three planes into the ring, an asynchronous copy per
+  // value, or zeros; lanes t, t + n, ...
+  auto load_row = [&](int row, int t, int n) {
+    if (row >= ny) return;
+    double* dst = ring + (unsigned)(row % kMailRows) * RL;
+    for (int p3 = 0; p3 < 3; p3++) {
+      const double* src = x + ((size_t)(k - 1 + p3) * ny + row) * nx;
+      for (int i = t; i < nx; i += n) {
+        double* d = dst + p3 * PS + (i & 1) * RUN + (i >> 1);
+        if (x_zero) {
+          *d = 0.0;
+        } else {
+          asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(
+                           (unsigned)__cvta_generic_to_shared(d)),
+                       "l"(src + i)
+                       : "memory");
+        }
+      }
     }
-    asm volatile("cp.async.wait_all;" ::: "memory");
-  }
-  __syncthreads();
+  };
+  if (has_plane)
+    for (int row = 0; row <= 3; row++) load_row(row, threadIdx.x, blockDim.x);
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  cl.sync();  // every inbox of the cluster is clear before anyone writes one
   const unsigned tag = tag_sh;
-  auto slot = [&](int plane_c, int q, int j, int m) -> unsigned long long* {
-    return mail + 2 * ((((size_t)plane_c * nhalf + q) * (ny - 2) + (j - 1)) * hr + m);
-  };
-  auto colour_i = [&](int j, int kk, int q, int m) -> int {
-    const int parity = (first_parity + q) & 1;
-    return 1 + (((1 + j + kk) & 1) != parity) + 2 * m;
-  };
-  // this thread's item: a fixed half-sweep (or the residual) and slot --
-  // threads [q hr, (q+1) hr) sweep half-sweep q, slot tid - q hr, threads
-  // from nhalf hr on the residual, point tid - nhalf hr -- at the row the
-  // step reaches: 0 = none, 1 = GS update, 2 = residual; j, i and, for a GS
-  // update, the slot m
-  const int iq = (int)threadIdx.x < nhalf * hr ? (int)threadIdx.x / hr : nhalf;
-  const int im = (int)threadIdx.x - iq * hr;
-  const bool iworker = iq < nhalf || (do_resid && im < nx - 2);
-  const int ilag = (iq < nhalf) ? wlag * iq : resid_lag;
-  auto item_of = [&](int s, int& j, int& i, int& q, int& m) -> int {
-    if (!iworker) return 0;
-    const int t = tmin + s - ilag;
-    const int jj = t - 2 * k;
-    if (t < tmin || t > tmax || jj < 1 || jj > ny - 2) return 0;
-    j = jj;
-    q = iq;
-    m = im;
-    if (iq < nhalf) {
-      i = colour_i(jj, k, iq, im);
-      return (i > nx - 2) ? 0 : 1;
-    }
-    i = 1 + im;
-    return 2;
-  };
-  // the mailbox slots this thread polls: thread group G = tid / hr takes the
-  // lower plane's half-sweep G (G < nhalf) or the upper plane's half-sweep
-  // G - nhalf, slot tid % hr, of row j+1 and, at j = 1, of row 1 too
-  const int grp = threadIdx.x / hr, gm = threadIdx.x - grp * hr;
-  const int pside = grp < nhalf ? 0 : 1;
-  const int pq = grp - pside * nhalf;
-  const int pph = pside == 0 ? pq : pq + 1;
-  const int pnb = pside == 0 ? c - 1 : c + 1;
-  const bool poller = grp < 2 * nhalf && pnb >= 0 && pnb < ncta && pph < nphase;
-  const int plag = (pph < nhalf) ? wlag * pph : resid_lag;
-  const unsigned long long* pp[kMailPoll];
-  double* dp[kMailPoll];
-  auto polls_of = [&](int s) -> unsigned {
-    unsigned pend = 0;
-    pp[0] = pp[1] = nullptr;
-    dp[0] = dp[1] = nullptr;
-    if (!poller) return 0;
-    const int t = tmin + s - plag;
-    const int j = t - 2 * k;
-    if (t < tmin || t > tmax || j < 1 || j > ny - 2) return 0;
-#pragma unroll
-    for (int pass = 0; pass < kMailPoll; pass++) {
-      const int jj = pass == 0 ? j + 1 : 1;
-      if (pass == 0 ? (jj > ny - 2) : (j != 1)) continue;
-      const int i = colour_i(jj, k - 1 + 2 * pside, pq, gm);
-      if (i > nx - 2) continue;
-      pp[pass] = slot(pnb, pq, jj, gm);
-      dp[pass] = (pside == 0 ? P0 : P2) + sidx(i, jj);
-      pend |= 1u << pass;
-    }
-    return pend;
-  };
+  const unsigned itag0 = tag * 64u + 1u;  // inbox tag of lap 0 (at most 127 / 8 laps)
   volatile int* verr = err;
-  unsigned long long w[kMailPoll][2];
-  auto issue = [&](unsigned pend) {
-#pragma unroll
-    for (int n = 0; n < kMailPoll; n++)
-      if (pend & (1u << n)) mail_load(pp[n], w[n][0], w[n][1]);
+  // a wait's bound: false once it ran out, here or elsewhere
+  auto keep_waiting = [&](unsigned long long& t0) -> bool {
+    if (failed_sh || *verr) {
+      failed_sh = 1;
+      return false;
+    }
+    const unsigned long long t = global_ns();
+    if (t0 == 0) t0 = t;
+    if ((long long)(t - t0) <= kWaveWaitNs) return true;
+    failed_sh = 1;
+    atomicAdd(err, 1);
+    return false;
   };
-  int j = 0, i = 0, q = 0, m = 0;
-  int kind = (nsteps > 0) ? item_of(0, j, i, q, m) : 0;
-  Coef27 C;
-  if (kind) load_coef27(op, cc, fc, g.idx(i, j, k), sy, sz, C);
-  // A step's polls are issued one step early, right after the previous
-  // step's barrier, so that their round trip overlaps that step's update:
-  // a slot that is already written then costs no wait at all.  (A plane's
-  // own loop -- poll round trip plus update -- sets the period of the plane
-  // below every other, and so of the whole wavefront.)
-  unsigned pend = (nsteps > 0) ? polls_of(0) : 0u;
-  issue(pend);
-  for (int s = 0; s < nsteps; s++) {
-    if (pend) {
-      const unsigned long long t0 = global_ns();
-      int spins = 0;
-      for (;;) {
+
+  if (!has_plane) {
+    // only the barriers
+  } else if ((int)threadIdx.x >= nwork + kMailCouriers) {
+    // ---- the loading warp: rows of x, and by lane q the coefficients of
+    // half-sweep q as the workers free their stages (bulk copies: they take no
+    // part of the load pipe that the workers' critical loads wait for)
+    const int lane = threadIdx.x & 31;
+    const int q = lane < nhalf ? lane : nhalf - 1;
+    int next = lane < nhalf ? 1 : ny;  // the next row of coefficients this lane copies
+    int xnext = 4, last = 0;
+    unsigned long long t0 = 0;
+    for (int spins = 1;; spins++) {
+      const int lim = min(ny - 2, max(0, prog_sh[q]) + NS);
+      for (; next <= lim; next++) {
+        const int st = (next - 1) % NS;
+        const unsigned bar = (unsigned)__cvta_generic_to_shared(&full[q][st]);
+        const double2* src =
+            pk + (((size_t)(k - 1) * (ny - 2) + (next - 1)) * 2 + ((first_parity + q) & 1)) * REC;
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar),
+                     "r"(REC * 16u)
+                     : "memory");
+        asm volatile(
+            "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, "
+            "[%3];" ::"r"((unsigned)__cvta_generic_to_shared(coef + (q * NS + st) * REC)),
+            "l"(src), "r"(REC * 16u), "r"(bar)
+            : "memory");
+        if (next + 4 <= ny - 2)
+          asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src + 8 * (size_t)REC),
+                       "r"(REC * 16u)
+                       : "memory");
+      }
+      __syncwarp();
+      // a row's slot is free once the last half-sweep's reads are above it
+      const int xlim = min(min(ny - 1, xnext + 3), prog_sh[nhalf - 1] + kMailRows - 2);
+      const int done = __shfl_sync(0xffffffffu, xlim, 0);
+      if (xnext <= done) {
+        for (; xnext <= done; xnext++) load_row(xnext, lane, 32);
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        __threadfence_block();
+        __syncwarp();
+        if (lane == 0) rows_sh = done;
+      }
+      if (__all_sync(0xffffffffu, xnext >= ny && next > ny - 2)) break;
+      const int at = xnext + __shfl_sync(0xffffffffu, next, 0);
+      if (at != last) {
+        last = at;
+        t0 = 0;
+      }
+      if ((spins & 63) == 0) {
+        int go = 1;
+        if (lane == 0) go = keep_waiting(t0);
+        if (!__shfl_sync(0xffffffffu, go, 0)) break;
+      }
+    }
+    // a copy must not outlive the CTA: those the workers did not wait for
+    // (after a failure) are waited for here
+    if (lane < nhalf)
+      for (int r = max(1, next - NS); r < next; r++) {
+        const unsigned bar = (unsigned)__cvta_generic_to_shared(&full[q][(r - 1) % NS]);
+        for (int n = 0; n < (1 << 20) && !mbar_done(bar, ((r - 1) / NS) & 1); n++) {
+        }
+      }
+  } else if ((int)threadIdx.x >= nwork) {
+    // ---- couriers: the foreign neighbour's global slots into the inbox
+    const int side = (rank == 0 && c > 0) ? 0 : ((rank == clsize - 1 && c + 1 < ncta) ? 1 : -1);
+    const int u = threadIdx.x - nwork;
+    const int nslot = side < 0 ? 0 : (side == 0 ? nhalf : nhalf - 1) * hr;
+    const int cn = side == 0 ? c - 1 : c + 1, kn = 1 + cn;
+    constexpr int kSlots = (kMailHalfMax * HP + kMailCouriers - 1) / kMailCouriers;
+    int row[kSlots], q[kSlots], m[kSlots];
 #pragma unroll
-        for (int n = 0; n < kMailPoll; n++) {
-          if ((pend & (1u << n)) && (unsigned)(w[n][0] >> 32) == tag &&
-              (unsigned)(w[n][1] >> 32) == tag) {
-            *dp[n] =
-                __longlong_as_double((long long)((w[n][1] << 32) | (w[n][0] & 0xffffffffull)));
-            pend &= ~(1u << n);
-          }
-        }
-        if (!pend) break;
-        if ((++spins & 15) == 0) {
-          if (failed_sh || *verr) {
-            failed_sh = 1;
-            break;
-          }
-          if ((long long)(global_ns() - t0) > kWaveWaitNs) {
-            failed_sh = 1;
-            atomicAdd(err, 1);
-            break;
-          }
-        }
-        issue(pend);
-      }
+    for (int n = 0; n < kSlots; n++) {
+      q[n] = (u + n * kMailCouriers) / hr;
+      m[n] = u + n * kMailCouriers - q[n] * hr;
     }
-    __syncthreads();
-    // the next step's polls go out now (the slots they fill are rows no
-    // update of this step reads, and they are copied in only after it)
-    pend = (s + 1 < nsteps) ? polls_of(s + 1) : 0u;
-    issue(pend);
-    if (kind) {
-      // the nine in-plane positions of the stencil (C: centre, N/S: j+-1,
-      // E/W: i+-1)
-      // (i +- 1 has the other parity: its run starts H further or H back,
-      // and its index in the run is i >> 1 or one less, plus the parity of i)
-      const int p = i & 1;
-      const int oC = sidx(i, j), oN = oC + 2 * H, oS = oC - 2 * H;
-      const int oE = oC + (1 - 2 * p) * H + p, oW = oE - 1;
-      const int oNE = oE + 2 * H, oNW = oW + 2 * H;
-      const int oSE = oE - 2 * H, oSW = oW - 2 * H;
-      const double tO = +C.o[0] * P1[oN] + C.o[1] * P1[oS] + C.o[2] * P1[oE] +
-                        C.o[3] * P1[oW] + C.o[4] * P1[oNE] + C.o[5] * P1[oNW] +
-                        C.o[6] * P1[oSE] + C.o[7] * P1[oSW];
-      const double tU = +C.u[0] * P2[oC] + C.u[1] * P2[oN] + C.u[2] * P2[oS] +
-                        C.u[3] * P2[oE] + C.u[4] * P2[oW] + C.u[5] * P2[oNE] +
-                        C.u[6] * P2[oNW] + C.u[7] * P2[oSE] + C.u[8] * P2[oSW];
-      const double tD = +C.d[0] * P0[oC] + C.d[1] * P0[oN] + C.d[2] * P0[oS] +
-                        C.d[3] * P0[oE] + C.d[4] * P0[oW] + C.d[5] * P0[oNE] +
-                        C.d[6] * P0[oNW] + C.d[7] * P0[oSE] + C.d[8] * P0[oSW];
-      if (kind == 1) {
-        const double v = (C.f + (tO + tU + tD)) / (C.oc + C.cc);
-        P1[oC] = v;
-        mail_put(slot(c, q, j, m), v, tag);
-      } else {
-        r[g.idx(i, j, k)] = C.f + tO + tU + tD - (C.oc + C.cc) * P1[oC];
+    // the first row from r on whose colour has this slot (odd nx: the last
+    // slot exists on every other row)
+    auto valid_from = [&](int n, int r) -> int {
+      const int b = (((1 + r + kn) & 1) != ((first_parity + q[n]) & 1)) ? 1 : 0;
+      return (1 + b + 2 * m[n] <= nx - 2) ? r : r + 1;
+    };
+#pragma unroll
+    for (int n = 0; n < kSlots; n++)
+      row[n] = u + n * kMailCouriers < nslot ? valid_from(n, 1) : ny;
+    unsigned long long t0 = 0;
+    for (int spins = 1;; spins++) {
+      unsigned long long w[kSlots][2][2];
+      int nrow[kSlots];
+      bool left = false;
+#pragma unroll
+      for (int n = 0; n < kSlots; n++) {
+        nrow[n] = ny;
+        if (row[n] > ny - 2) continue;
+        left = true;
+        nrow[n] = valid_from(n, row[n] + 1);
+        const unsigned long long* p0 =
+            mail + 2 * ((((ptrdiff_t)cn * nhalf + q[n]) * (ny - 2) - 1) * hr + m[n]);
+        mail_load(p0 + 2 * (size_t)row[n] * hr, w[n][0][0], w[n][0][1]);
+        if (nrow[n] <= ny - 2) mail_load(p0 + 2 * (size_t)nrow[n] * hr, w[n][1][0], w[n][1][1]);
       }
+      if (!left) break;
+#pragma unroll
+      for (int n = 0; n < kSlots; n++) {
+#pragma unroll
+        for (int d = 0; d < 2; d++) {
+          if (row[n] > ny - 2 || (d == 1 && row[n] != nrow[n])) break;
+          if (!mail_is(w[n][d][0], w[n][d][1], tag)) break;
+          const unsigned long long it =
+              (unsigned long long)(itag0 + (unsigned)row[n] / kMailInRows) << 32;
+          unsigned long long* s = inbox + (side * kMailHalfMax + q[n]) * IBOX +
+                                  (row[n] & (kMailInRows - 1)) * IROW + 2 * m[n];
+          inbox_put((unsigned)__cvta_generic_to_shared(s), (w[n][d][0] & 0xffffffffull) | it,
+                    (w[n][d][1] & 0xffffffffull) | it);
+          row[n] = d == 0 ? nrow[n] : valid_from(n, row[n] + 1);
+          t0 = 0;
+        }
+      }
+      if ((spins & 63) == 0 && !keep_waiting(t0)) break;
     }
-    // the next step's coefficients do not depend on this step: fetch them
-    // while the neighbour planes finish
-    const int nkind = (s + 1 < nsteps) ? item_of(s + 1, j, i, q, m) : 0;
-    if (nkind) load_coef27(op, cc, fc, g.idx(i, j, k), sy, sz, C);
-    kind = nkind;
+  } else {
+    // ---- workers: this thread's half-sweep, slot and colour
+    const int width = nwork / nhalf;
+    const int q = threadIdx.x / width, m = threadIdx.x - q * width;
+    const int par = (first_parity + q) & 1;
+    // the points of row j are i = 1 + b + 2m, b alternating from row to row;
+    // the last slot of a row with b = 1 is empty.  The lower plane's row j+1
+    // and the upper plane's row j+2 (of the other colour) have the same i.
+    const bool on[2] = {m < hr, m < hr - 1};
+    const bool has_lo = c > 0, has_up = c + 1 < ncta && q > 0;
+    // (lanes beyond the row poll slot 0, without use)
+    const unsigned in_lo =
+        (unsigned)__cvta_generic_to_shared(inbox + q * IBOX + 2 * (m < HP ? m : 0));
+    const unsigned in_up = (unsigned)__cvta_generic_to_shared(
+        inbox + (kMailHalfMax + (q > 0 ? q - 1 : 0)) * IBOX + 2 * (m < HP ? m : 0));
+    // where this thread's updates go: the upper plane's inbox, the lower
+    // plane's (if a later half-sweep reads them there), the global slot
+    const bool to_up = c + 1 < ncta, to_lo = c > 0 && q + 1 < nhalf;
+    const bool in_cl_up = to_up && rank + 1 < clsize, in_cl_lo = to_lo && rank > 0;
+    const bool to_global = (to_up && !in_cl_up) || (to_lo && !in_cl_lo);
+    const bool to_x = q >= nhalf - 2;
+    const unsigned out_up = in_cl_up ? cluster_addr(inbox + q * IBOX + 2 * m, rank + 1) : 0u;
+    const unsigned out_lo =
+        in_cl_lo ? cluster_addr(inbox + (kMailHalfMax + q) * IBOX + 2 * m, rank - 1) : 0u;
+    unsigned long long* own =  // slot of row j, which starts at -1
+        mail + 2 * ((((ptrdiff_t)c * nhalf + q) * (ny - 2) - 2) * hr + m);
+    // row j of x at column 1 + 2m, row j + 2 of f
+    double* xrow = x + ((ptrdiff_t)k * ny - 1) * nx + 1 + 2 * m;
+    const double* frow = fc + (ptrdiff_t)k * ny * nx + 1 + 2 * m;
+    // the stage of row j + 1's coefficients, with the parity of its barrier
+    const double2* cst = coef + q * NS * REC + m;
+    const unsigned bar0 = (unsigned)__cvta_generic_to_shared(&full[q][0]);
+    unsigned stage = 0, parity = 0;
+    // ring offsets of rows j-1, j, j+1 at slot m; inbox rows j, j+1 (byte
+    // offset and tag)
+    auto next_row = [&](unsigned o) -> unsigned {
+      return o + RL >= PS + (unsigned)m ? o + RL - PS : o + RL;
+    };
+    unsigned om = (kMailRows - 2) * RL + m, o0 = (kMailRows - 1) * RL + m, op = m;  // j = -1
+    unsigned ia = (kMailInRows - 1) * (8u * IROW), ib = 0, ta = itag0 - 1u, tb = itag0;
+    volatile int* prev = &prog_sh[q > 0 ? q - 1 : 0];
+    volatile int* follow = &prog_sh[q + 1 < nhalf ? q + 1 : q];
+    double fnext = 0.0;  // f of row j + 1
+    // f of the row frow is at (B: its colour offset), then on to the next
+    auto fetch = [&](auto bsel, int j) {
+      constexpr int B = decltype(bsel)::value;
+      if (on[B] && (unsigned)(j - 1) < (unsigned)(ny - 2)) fnext = __ldg(frow + B);
+      frow += nx;
+    };
+    // step j (row j, colour offset B)
+    auto step = [&](auto bsel, int j, Ready27& R) {
+      constexpr int B = decltype(bsel)::value;
+      constexpr int oc = B == 0 ? RUN : 1, oe = B == 0 ? 1 : RUN + 1;      // row j's columns
+      constexpr int nc = B == 0 ? 1 : RUN, ne = B == 0 ? RUN + 1 : 1;      // row j+1's
+      const unsigned on2 = next_row(op);                                   // row j+2
+      const unsigned ic = ib + 8u * IROW == 8u * IBOX ? 0u : ib + 8u * IROW;
+      const unsigned tc = ic == 0u ? tb + 1u : tb;
+      // what the step waits for: its mail; for its end rows of x, coefficients
+      // and the half-sweep before it three rows ahead; the one after it within
+      // wlag rows.  The loads are issued together.
+      const bool lo = has_lo && on[B] && (unsigned)j < (unsigned)(ny - 2);
+      const bool up = has_up && on[B] && (unsigned)(j + 1) < (unsigned)(ny - 2);
+      const bool prep = (unsigned)j < (unsigned)(ny - 2);
+      const int want = min(j + 2, ny - 1);
+      const int ahead = q > 0 && prep ? min(j + 3, ny - 1) : -2;
+      const int behind = q + 1 < nhalf ? j - wlag : -2;
+      const unsigned bar = bar0 + 8u * stage;
+      unsigned long long w0, w1, v0, v1, t0 = 0;
+      for (int spins = 1;; spins++) {
+        inbox_load(in_lo + ib, w0, w1);
+        inbox_load(in_up + ic, v0, v1);
+        const int rows = rows_sh, pa = *prev, pb = *follow;
+        const bool there = mbar_done(bar, parity);
+        if ((!lo || mail_is(w0, w1, tb)) && (!up || mail_is(v0, v1, tc)) && rows >= want &&
+            pa >= ahead && pb >= behind && (there || !prep))
+          break;
+        if ((spins & 255) == 0 && !keep_waiting(t0)) break;
+      }
+      if (lo) ring[op + oc] = __longlong_as_double((long long)((w1 << 32) | (unsigned)w0));
+      if (up)
+        ring[2 * PS + on2 + oc] = __longlong_as_double((long long)((v1 << 32) | (unsigned)v0));
+      // the threads of the half-sweep
+      if (width == 32) __syncwarp();
+      else asm volatile("bar.sync %0, %1;" ::"r"(1 + q), "r"(width) : "memory");
+      if (m == 0) prog_sh[q] = j;
+      if (on[B] && (unsigned)(j - 1) < (unsigned)(ny - 2)) {
+        // the late neighbours, the rest of the sums in the reference's order
+        const double tD = R.d0 + R.a1 * ring[op + oc] + R.d2 + R.d3 + R.d4 + R.d5 + R.d6 + R.d7 +
+                          R.d8;
+        const double tO = R.o + R.a6 * ring[PS + om + oe] + R.a7 * ring[PS + om + oe - 1];
+        const double v = div_by(R.f + (tO + R.u + tD), R.diag, R.rdiag);
+        const unsigned long long bits = (unsigned long long)__double_as_longlong(v);
+        const unsigned long long it = (unsigned long long)ta << 32;
+        const unsigned long long w0 = (bits & 0xffffffffull) | it, w1 = (bits >> 32) | it;
+        if (in_cl_up) inbox_put(out_up + ia, w0, w1);
+        if (in_cl_lo) inbox_put(out_lo + ia, w0, w1);
+        if (to_global) mail_put(own, v, tag);
+        ring[PS + o0 + oc] = v;
+        if (to_x) __stcg(xrow + B, v);
+      }
+      own += 2 * hr;
+      xrow += nx;
+      om = o0;
+      o0 = op;
+      op = on2;
+      ia = ib;
+      ib = ic;
+      ta = tb;
+      tb = tc;
+      // the next row's early products, from its coefficients
+      if (prep) {
+        if (on[1 - B]) {
+          const double2* cp = cst + stage * REC;
+          const double* rm = ring + om;
+          const double* r0 = ring + o0;
+          const double* rp = ring + op;
+          auto K = [&](int t) -> double2 { return cp[t * HP]; };
+          const double2 k0 = K(0), k1 = K(1), k2 = K(2), k3 = K(3), k4 = K(4), k5 = K(5),
+                        k6 = K(6), k7 = K(7), k8 = K(8), k9 = K(9), k10 = K(10), k11 = K(11),
+                        k12 = K(12), k13 = K(13);
+          R.o = +k0.x * rp[PS + nc] + k0.y * rm[PS + nc] + k1.x * r0[PS + ne] +
+                k1.y * r0[PS + ne - 1] + k2.x * rp[PS + ne] + k2.y * rp[PS + ne - 1];
+          R.u = +k4.x * r0[2 * PS + nc] + k4.y * rp[2 * PS + nc] + k5.x * rm[2 * PS + nc] +
+                k5.y * r0[2 * PS + ne] + k6.x * r0[2 * PS + ne - 1] + k6.y * rp[2 * PS + ne] +
+                k7.x * rp[2 * PS + ne - 1] + k7.y * rm[2 * PS + ne] + k8.x * rm[2 * PS + ne - 1];
+          R.d0 = k8.y * r0[nc];
+          R.d2 = k9.y * rm[nc];
+          R.d3 = k10.x * r0[ne];
+          R.d4 = k10.y * r0[ne - 1];
+          R.d5 = k11.x * rp[ne];
+          R.d6 = k11.y * rp[ne - 1];
+          R.d7 = k12.x * rm[ne];
+          R.d8 = k12.y * rm[ne - 1];
+          R.a1 = k9.x;
+          R.a6 = k3.x;
+          R.a7 = k3.y;
+          R.f = fnext;
+          R.diag = k13.x;
+          R.rdiag = k13.y;
+        }
+        stage++;
+        if (stage == NS) {
+          stage = 0;
+          parity ^= 1u;
+        }
+      }
+      fetch(bsel, j + 2);
+    };
+
+    // row -1 has colour offset b0; the loop starts with an offset-0 step,
+    // skipped (j = -2) where row -1 has offset 1.  The last step only says
+    // that row ny - 2 is updated.
+    const std::integral_constant<int, 0> B0{};
+    const std::integral_constant<int, 1> B1{};
+    const int b0 = ((k & 1) != par) ? 1 : 0;
+    Ready27 R;
+    if (b0) fetch(B0, 0);
+    else fetch(B1, 0);
+    for (int j = -1 - b0; j <= ny - 1; j += 2) {
+      if (j >= -1) step(B0, j, R);
+      if (j + 1 <= ny - 1) step(B1, j + 1, R);
+    }
+    if (threadIdx.x == 0) counters[c] = tag;
   }
-  __syncthreads();
-  double* dst = x + (size_t)k * pn;
-  for (int e = threadIdx.x; e < pn; e += blockDim.x) {
-    const int jj = e / nx, ii = e - jj * nx;
-    if (jj >= 1 && jj <= ny - 2 && ii >= 1 && ii <= nx - 2) __stcg(dst + e, P1[sidx(ii, jj)]);
-  }
-  if (threadIdx.x == 0) counters[c] = tag;
+  cl.sync();  // no CTA exits while a neighbour may write its inbox
 }
 
-int wave_mail_fit(Grid g) {
-  static int dev_smem = -1, sms = 0;
-  if (dev_smem < 0) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&dev_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+using MailKernel = void (*)(Grid, const double2*, const double*, double*, int, int, int,
+                            unsigned*, int*, int, unsigned long long*);
+static MailKernel mail_kernel(Grid g) {
+  switch (pack_hr(g)) {
+    case 8: return k_gs27_mail<8>;
+    case 16: return k_gs27_mail<16>;
+    case 24: return k_gs27_mail<24>;
+    case 32: return k_gs27_mail<32>;
+    case 40: return k_gs27_mail<40>;
+    case 48: return k_gs27_mail<48>;
+    case 56: return k_gs27_mail<56>;
+    default: return nullptr;
   }
+}
+
+// The launch of a level: the largest cluster that the device can hold all the
+// planes with at once (fewest hand-overs through global memory).
+struct MailPlan {
+  MailKernel kernel = nullptr;  // nullptr: the level does not fit
+  int cluster = 0, threads = 0;
+  size_t smem = 0;
+};
+static MailPlan mail_plan(Grid g, int nhalf) {
+  MailPlan p;
   const int planes = g.nz - 2;
-  const int hr = (g.nx - 1) / 2;
-  const int items = kMailHalfMax * hr + (g.nx - 2);
-  const int pollers = 2 * kMailHalfMax * hr;
-  const size_t smem = mail_smem(g);
-  return planes >= 2 && planes <= kWavePlanesMax && planes <= sms && items <= kMailThreads &&
-         pollers <= kMailThreads && smem + 1024 <= (size_t)dev_smem;
+  const MailKernel kernel = mail_kernel(g);
+  p.threads = nhalf * ((mail_hr(g) + 31) / 32 * 32) + kMailHelpers;
+  p.smem = mail_smem(g);
+  int dev = 0, lim = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&lim, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  if (!kernel || planes < 2 || planes > kWavePlanesMax || p.smem + 1024 > (size_t)lim) return p;
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem) !=
+          cudaSuccess ||
+      cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) !=
+          cudaSuccess) {
+    cudaGetLastError();
+    return p;
+  }
+  for (int n = 16; n >= 2 && !p.kernel; n /= 2) {
+    if (n > 2 && n / 2 >= planes) continue;
+    const int clusters = (planes + n - 1) / n;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(clusters * n, 1, 1);
+    cfg.blockDim = dim3(p.threads, 1, 1);
+    cfg.dynamicSmemBytes = p.smem;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = n;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    int fit = 0;
+    if (cudaOccupancyMaxActiveClusters(&fit, kernel, &cfg) == cudaSuccess && fit >= clusters) {
+      p.kernel = kernel;
+      p.cluster = n;
+    }
+    cudaGetLastError();
+  }
+  return p;
 }
 
-int launch_gs27_mail(cudaStream_t s, Grid g, Op op, const double* cc, const double* fc,
-                     double* x, double* r, int nsweep, int first_parity, unsigned* counters,
-                     int* err, int wlag, unsigned long long* mail) {
-  int nhalf = 2 * nsweep;
-  int do_resid = (r != nullptr) ? 1 : 0;
-  if (!mail || nhalf < 2 || nhalf > kMailHalfMax || !wave_mail_fit(g)) return 0;
-  const int hr = (g.nx - 1) / 2;
-  const int items = nhalf * hr + (do_resid ? g.nx - 2 : 0);
-  int threads = std::max(items, 2 * nhalf * hr);
-  threads = std::max(64, (threads + 31) / 32 * 32);
-  if (threads > kMailThreads) return 0;
-  const size_t smem = mail_smem(g);
-  static size_t smem_set = 0;
-  if (smem > smem_set) {
-    if (cudaFuncSetAttribute(k_gs27_mail, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)smem) != cudaSuccess)
-      return 0;
-    smem_set = smem;
-  }
-  int per_sm = 0, sms = 0, dev = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_gs27_mail, threads, smem) !=
-          cudaSuccess ||
-      per_sm * sms < g.nz - 2)
-    return 0;
-  if (wlag < 4) wlag = 4;
-  void* args[] = {&g, &op, &cc, &fc, &x, &r, &nhalf, &first_parity, &do_resid,
-                  &counters, &err, &wlag, &mail};
-  return cudaLaunchCooperativeKernel((void*)k_gs27_mail, dim3(g.nz - 2), dim3(threads), args,
-                                     smem, s) == cudaSuccess;
+int wave_mail_fit(Grid g) { return mail_plan(g, kMailHalfMax).kernel != nullptr; }
+
+int launch_gs27_mail(cudaStream_t s, Grid g, const double* pack, const double* fc, double* x,
+                     int x_zero, int nsweep, int first_parity, unsigned* counters, int* err,
+                     int wlag, unsigned long long* mail) {
+  const int nhalf = 2 * nsweep;
+  if (!mail || !pack || nhalf < 3 || nhalf > kMailHalfMax) return 0;
+  const MailPlan p = mail_plan(g, nhalf);
+  if (!p.kernel) return 0;
+  wlag = std::min(std::max(wlag, 4), kMailLagMax);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((g.nz - 2 + p.cluster - 1) / p.cluster * p.cluster, 1, 1);
+  cfg.blockDim = dim3(p.threads, 1, 1);
+  cfg.dynamicSmemBytes = p.smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at[2];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = p.cluster;
+  at[0].val.clusterDim.y = 1;
+  at[0].val.clusterDim.z = 1;
+  at[1].id = cudaLaunchAttributeCooperative;  // the planes wait on one another
+  at[1].val.cooperative = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 2;
+  return cudaLaunchKernelEx(&cfg, p.kernel, g, reinterpret_cast<const double2*>(pack), fc, x,
+                            x_zero, nhalf, first_parity, counters, err, wlag, mail) ==
+         cudaSuccess;
 }
 
 int mg_init() {

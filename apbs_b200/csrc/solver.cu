@@ -362,14 +362,21 @@ extern "C" int pmgb_create(const pmgb_params* params, int precision, pmgb_solver
   if (ok) ok &= (cudaMemset(s->d_wave, 0, kWaveWords * sizeof(unsigned)) == cudaSuccess);
   // mailboxes for the levels the ordered GS27 smooths (all but the
   // coarsest) where the shared-memory plane wavefront fits
+  // (the mixed path does not run it)
   s->mail_total = 0;
+  size_t pack_total = 0;
   for (int l = 0; l < 12; l++) {
     s->mail_off[l] = -1;
-    if (l >= 1 && l < s->nlev - 1 && wave_mail_fit(s->lev[l].g)) {
+    if (precision == PMGB_FP64 && l >= 1 && l < s->nlev - 1 && wave_mail_fit(s->lev[l].g)) {
       s->mail_off[l] = (long long)s->mail_total;
       s->mail_total += mail_words(s->lev[l].g);
+      s->pack_off[l] = pack_total;
+      pack_total += gs27_pack_doubles(s->lev[l].g);
     }
   }
+  // written by gs27_pack before its first use
+  if (ok && pack_total)
+    ok &= (cudaMalloc(&s->d_pack, pack_total * sizeof(double)) == cudaSuccess);
   if (ok && s->mail_total) {
     ok &= (cudaMalloc(&s->d_mail, s->mail_total * sizeof(unsigned long long)) == cudaSuccess);
     if (ok)
@@ -513,12 +520,13 @@ extern "C" size_t pmgb_footprint(const pmgb_params* params, int precision, int n
   for (int l = 0; l < nlev; l++) d += (size_t)((l == 0 ? 4 : 14) + 7) * nl[l];
   size_t bytes = d * sizeof(double);
   bytes += 3 * n;  // the dielectric byte maps
-  // mailboxes of the shared-memory GS27 wavefront (levels whose three planes
-  // fit in a CTA's shared memory; an upper bound where the device says no)
-  for (int l = 1; l < nlev - 1; l++)
-    if ((size_t)3 * gx[l] * gy[l] * sizeof(double) + 1024 <= 232448)
-      bytes += 2 * sizeof(unsigned long long) * (size_t)(gz[l] - 2) * 4 * (gy[l] - 2) *
-               ((gx[l] - 1) / 2);
+  // mailboxes and packed coefficients of the FP64 plane wavefront (an upper
+  // bound where the device has fewer SMs than the level planes)
+  for (int l = 1; precision == PMGB_FP64 && l < nlev - 1; l++)
+    if (gx[l] <= 113) {
+      const Grid g{gx[l], gy[l], gz[l]};
+      bytes += mail_words(g) * sizeof(unsigned long long) + gs27_pack_doubles(g) * sizeof(double);
+    }
   // FP32 hierarchy from level lo, plus Galerkin levels down to <= 512 unknowns
   const int lo = (precision == PMGB_MIXED) ? 0 : nlev - 1;
   const size_t nc_int = (size_t)(gx[nlev - 1] - 2) * (gy[nlev - 1] - 2) * (gz[nlev - 1] - 2);
@@ -569,6 +577,7 @@ extern "C" void pmgb_destroy(pmgb_solver* s) {
   dfree(s->nw_r0); dfree(s->nw_ws); dfree(s->nw_keepx); dfree(s->nw_keepr);
   dfree(s->part); dfree(s->scal); dfree(s->d_iters); dfree(s->d_info); dfree(s->d_npts); dfree(s->d_wave); dfree(s->d_forces);
   if (s->d_mail) cudaFree(s->d_mail);
+  if (s->d_pack) cudaFree(s->d_pack);
   dfree(s->d_opptrs);
   dfree(s->band);
   dfree(s->focus_w);
@@ -969,6 +978,7 @@ static int build_ops(pmgb_solver* s) {
     launch_restrict(st, P.g, P.fc, C.g, C.fc);
     note_launches(3);
   }
+  s->pack_cc = 0;  // the packed coefficients are made again before their next use
   // the mixed-precision path re-derives its FP32 hierarchy from these
   if (s->mixed) mixed_mark_stale(s->mixed);
   // coarsest direct solve for the linear problem (Vbuildband, buildBd.c:57-117);
@@ -1013,21 +1023,50 @@ int pmgb::solver_build(pmgb_solver* s) { return build_ops(s); }
 // ===========================================================================
 // one V-cycle (body of the do-loop of Vmvcs, src/pmgc/mgcsd.c:312-562)
 // ===========================================================================
-// ordered 27-point smoothing of level l (two sweeps, optional residual):
-// the plane-parallel wavefront on every level that fits it, else the
-// one-cluster wavefront (PMGB_TUNE_GS27_PLANES = 1: always the latter)
+// the packed coefficients of the levels the mailbox wavefront smooths, with
+// the Helmholtz terms cc (linear system) or cp (Newton system); after the
+// operators were rebuilt or the Newton term was
+static void gs27_pack(pmgb_solver* s, int newton) {
+  if (!s->d_pack || s->tune[PMGB_TUNE_GS27_PLANES] != 0) return;
+  const int want = newton ? 2 : 1;
+  if (!newton && s->pack_cc == want) return;
+  for (int l = 1; l < s->nlev - 1; l++) {
+    const Level& L = s->lev[l];
+    if (s->mail_off[l] < 0) continue;
+    launch_gs27_pack(s->stream, L.g, L.ops(), newton ? L.cp : L.cc, s->d_pack + s->pack_off[l],
+                     s->pack_cc == 0);
+    note_launches(1);
+  }
+  s->pack_cc = want;
+}
+
+// ordered 27-point smoothing of level l (two sweeps; x_zero: from x = 0), then
+// the residual where r is given: the mailbox wavefront on every level that
+// fits it, else the step-counter one, else the one-cluster wavefront
+// (PMGB_TUNE_GS27_PLANES = 1: always the last).  k counts the kernels launched.
 static int gs27_smooth(pmgb_solver* s, cudaStream_t st, int l, const double* cc,
-                       const double* fc, double* x, double* r, int first_parity) {
+                       const double* fc, double* x, int x_zero, double* r, int first_parity,
+                       long long& k) {
   const Level& L = s->lev[l];
   if (s->tune[PMGB_TUNE_GS27_PLANES] == 0 && s->mail_off[l] >= 0 &&
-      launch_gs27_mail(st, L.g, L.ops(), cc, fc, x, r, 2, first_parity,
+      launch_gs27_mail(st, L.g, s->d_pack + s->pack_off[l], fc, x, x_zero, 2, first_parity,
                        s->d_wave + kWaveCounterBase + (size_t)l * kWavePlanesMax,
                        reinterpret_cast<int*>(s->d_wave), s->tune[PMGB_TUNE_GS27_LAG],
                        s->d_mail + s->mail_off[l])) {
     s->wave_used = 1;
+    k++;
+    if (r) {
+      launch_resid(st, L.g, L.ops(), cc, fc, x, r);
+      k++;
+    }
     return 1;
   }
   (void)cudaGetLastError();  // a refused launch above leaves no error behind
+  if (x_zero) {
+    launch_zero(st, x, L.g.n());
+    k++;
+  }
+  k++;
   if (s->tune[PMGB_TUNE_GS27_PLANES] != 1 && wave_planes_fit(L.g)) {
     s->wave_used = 1;
     return launch_gs27_planes(st, L.g, L.ops(), cc, fc, x, r, 2, first_parity,
@@ -1075,13 +1114,9 @@ static int vcycle_body(pmgb_solver* s, int newton) {
     Level& P = s->lev[l - 1];
     launch_restrict(st, P.g, s->w1, C.g, C.w0);
     k++;
-    if (l != nlev - 1) {
-      launch_zero(st, X(l), C.g.n());
-      if (!gs27_smooth(s, st, l, CC(l), C.w0, X(l), s->w1, 1)) {
-        set_error("gs27 launch failed at level %d", l);
-        return 0;
-      }
-      k += 2;
+    if (l != nlev - 1 && !gs27_smooth(s, st, l, CC(l), C.w0, X(l), 1, s->w1, 1, k)) {
+      set_error("gs27 launch failed at level %d", l);
+      return 0;
     }
   }
   // coarsest
@@ -1130,11 +1165,10 @@ static int vcycle_body(pmgb_solver* s, int newton) {
         k += 2;
       }
     } else {
-      if (!gs27_smooth(s, st, l, CC(l), P.w0, X(l), nullptr, 0)) {
+      if (!gs27_smooth(s, st, l, CC(l), P.w0, X(l), 0, nullptr, 0, k)) {
         set_error("gs27 launch failed at level %d", l);
         return 0;
       }
-      k++;
     }
   }
   // stopping test residual
@@ -1181,6 +1215,7 @@ static int vcycles(pmgb_solver* s, int newton, double errtol, int itmax, int ist
   if (rsden == 0.0) rsden = 1.0;
   rsnrm = rsden;
   s->reslog.push_back(rsnrm / rsden);
+  gs27_pack(s, newton);
   if (!ensure_graph(s, newton)) return 0;
   int iters = 0;
   do {
@@ -1563,6 +1598,7 @@ extern "C" int pmgb_time_kernel(pmgb_solver* s, int which, int reps, double* ms,
   const double fint = (double)(F.g.nx - 2) * (F.g.ny - 2) * (F.g.nz - 2);
   double b = 0.0;
   if (which == PMGB_K_GS7_SWEEP_FP32 && !mixed_prepare_sweep(s)) return 0;
+  if (which == PMGB_K_GS27_WAVE) gs27_pack(s, 0);
   CK(cudaStreamSynchronize(st));
   CK(cudaEventRecord(s->ev[6], st));
   for (int r = 0; r < reps; r++) {
@@ -1576,8 +1612,8 @@ extern "C" int pmgb_time_kernel(pmgb_solver* s, int which, int reps, double* ms,
         if (s->nlev < 3) { set_error("pmgb_time_kernel: needs >= 3 levels"); return 0; }
         Level& C = s->lev[1];
         const double cint = (double)(C.g.nx - 2) * (C.g.ny - 2) * (C.g.nz - 2);
-        if (!gs27_smooth(s, st, 1, C.cc, C.w0, C.x, s->w1, 1))
-          return 0;
+        long long kernels = 0;
+        if (!gs27_smooth(s, st, 1, C.cc, C.w0, C.x, 0, s->w1, 1, kernels)) return 0;
         // 14 coefficients + cc + f read, x read and written: 144 B per point
         // per sweep; the residual pass reads the same and writes r
         b = (2.0 * 144.0 + 144.0) * cint;

@@ -141,6 +141,11 @@ struct pmgb_solver {
   unsigned long long* d_mail;
   long long mail_off[12];
   size_t mail_total;
+  // FP64 only: packed coefficients of the same levels (launch_gs27_pack);
+  // pack_cc: the Helmholtz terms their diagonals hold (0 none yet, 1 cc, 2 cp)
+  double* d_pack;
+  size_t pack_off[12];
+  int pack_cc;
   double* atom_terms;  // 13 x natoms sdh moment terms
   size_t terms_alloc;
   // focusing: faces set from a coarse solution, energies outside the domain

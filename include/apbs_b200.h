@@ -222,8 +222,9 @@ int pmgb_solve_molecule(const pmgb_params *params, int precision, int natoms,
                                           sweeps), K > 0 = Jacobi-preconditioned Chebyshev of
                                           degree K (rounded up to even) */
 #define PMGB_TUNE_GS27_LAG 1          /* plane-parallel GS27: wavefronts between successive
-                                          half-sweeps (>= 4, default 6); a larger lag lets a
-                                          plane run ahead of the plane above it */
+                                          half-sweeps (>= 4, default 6; the mailbox kernel
+                                          takes at most 6); a larger lag lets a plane run
+                                          ahead of the plane above it */
 /* key 3 is not used */
 #define PMGB_TUNE_GS27_CLUSTER 2       /* CTAs per cluster of the ordered GS27 on levels with
                                           >= 60 interior points per axis (0 = device max) */
@@ -251,9 +252,11 @@ int pmgb_solve_molecule(const pmgb_params *params, int precision, int natoms,
                                           of 2 x (slots - nx - 3) points of each plane;
                                           default 0x12: 1024 threads, 1 slot */
 #define PMGB_TUNE_GS27_PLANES 13      /* ordered GS27: 0 (default) = one CTA per plane
-                                          holding its plane and both neighbours in shared
-                                          memory, updates passed through a mailbox, on
-                                          levels where three planes fit (else as 2);
+                                          holding rows of its plane and both neighbours in
+                                          shared memory, updates passed by value through
+                                          cluster shared memory or a mailbox, on levels of
+                                          up to 113 points along x whose planes fit on the
+                                          device (else as 2);
                                           2 = one CTA per plane synchronised with its
                                           neighbour planes by step counters on every level
                                           whose planes fit on the device; 1 = one cluster
