@@ -902,20 +902,22 @@ int launch_gs27_planes(cudaStream_t s, Grid g, Op op, const double* cc, const do
 // neighbour's use of it.  A global slot (k, q, j, m) is written once per
 // launch and tagged with the launch count of its plane.  The slots in shared
 // memory (the inbox) are a ring over the rows, tagged with the launch and the
-// lap; a neighbour is never more than wlag rows ahead of its reader (below),
-// and the ring holds wlag + 2.
+// lap; a neighbour is at most wlag - 1 rows ahead of its reader (below), which is
+// what the ring holds.
 //
-// Each half-sweep q of a plane has its own warps, which go through its rows in
-// steps.  Step j first takes mail into the CTA's copies of the neighbour planes
-// -- row j+1 of the lower plane's half-sweep q, and for the next step row j+2 of
-// the upper plane's half-sweep q-1 -- then updates row j.  A half-sweep follows
-// the one before it on its plane by at least three rows and at most wlag.  The
-// rows an update reads hold exactly the values the sequential order reads (the
-// lower plane swept by this half-sweep, the upper one by the earlier ones), and
-// the rows a step changes lie outside those any other half-sweep may still
-// read.  The iterates are bitwise those of k_gs27_wave whatever the order in
-// which planes and half-sweeps run; tests/test_gs27_mail_ring.py runs this rule
-// on adversarial interleavings, and how far a neighbour gets ahead.
+// Each half-sweep q of a plane has two groups of threads, one for the rows of
+// either parity.  For its row j a group takes row j+1 of the upper plane's
+// half-sweep q-1 from the inbox, makes the products that need no late neighbour,
+// takes row j+1 of the lower plane's half-sweep q, and updates the row: the late
+// neighbours are that mail, the lower plane's row j and this plane's row j-1,
+// which the other group has just dealt with.  A half-sweep follows the one before
+// it on its plane by at least two rows and at most wlag.  The rows an update
+// reads hold exactly the values the sequential order reads (the lower plane swept
+// by this half-sweep, the upper one by the earlier ones), and the rows it changes
+// lie outside those any other half-sweep may still read.  The iterates are
+// bitwise those of k_gs27_wave whatever the order in which planes, half-sweeps
+// and groups run; tests/test_gs27_mail_ring.py runs this rule on adversarial
+// interleavings, and how far a neighbour gets ahead.
 //
 // What bounds it: the wave reaches plane k two steps and one hand-over after
 // plane k-1, so its length is (planes) x (step + hand-over) + (rows) x step.
@@ -923,10 +925,11 @@ int launch_gs27_planes(cudaStream_t s, Grid g, Op op, const double* cc, const do
 // round trip, about as much as the rest of a step; a store to a neighbour SM's
 // shared memory and a poll of the own one cost a fraction of it.  The rest of
 // the step is kept short:
-//  * Only three of the 26 neighbours change in the step before an update (the
-//    lower plane's (i, j+1) and the own plane's (i+-1, j-1)).  The other 23
-//    products, and the sums that precede them in the reference's order, are
-//    made at the end of the previous step, after its updates were sent.
+//  * Only five of the 26 neighbours change in the row before (the lower plane's
+//    (i, j+1) and (i+-1, j), the own plane's (i+-1, j-1)).  The other products,
+//    and the sums that precede them in the reference's order, are made while the
+//    other group updates its row: a single warp takes about 1700 cycles for all
+//    of a row's instructions, of which the late part is a third.
 //  * Coefficients in the order an update reads them (k_gs27_pack): per row and
 //    colour, 14 pairs of doubles for each point, contiguous over the points of
 //    the colour -- the 26 couplings, the diagonal D = oC + cc and 1/D.  Read
@@ -935,21 +938,22 @@ int launch_gs27_planes(cudaStream_t s, Grid g, Op op, const double* cc, const do
 //    copies, which take no part of the load pipe the workers' critical loads
 //    wait for.
 //  * A ring of rows of the three planes instead of whole planes (nx up to 113
-//    instead of 97), loaded by the same warp.
+//    instead of 97), loaded by another warp.
 //  * Half-sweeps are not in lockstep: one's waits overlap another's products.
 //  * The last two half-sweeps store their updates to x themselves, so nothing
 //    follows the last step; an iterate known to be zero is neither written nor
 //    loaded.
 //  * A quotient by the prefetched reciprocal, correctly rounded (div_by).
-//  * At the edge of a cluster, couriers (four warps) poll the foreign
+//  * At the edge of a cluster, couriers (two warps) poll the foreign
 //    neighbour's global slots, two rows at a time, and put the values into the
 //    inbox: the polls' round trips are off the workers' path.
 //  * The residual is a kernel of its own: it would double the loads of a step
 //    for a pass that needs no order.
-// Measured (two sweeps and the residual, lag 6; in brackets the kernels before,
-// whole planes in shared memory and a global mailbox, at 113^3 step counters):
-// 17^3 49 us (66), 33^3 96 (126), 49^3 150 (203), 65^3 212 (289), 81^3 300 (455),
-// 97^3 460 (744), 113^3 558 (1244).
+// Measured (two sweeps and the residual; in brackets the kernels before, whole
+// planes in shared memory and a global mailbox, at 113^3 step counters):
+// 17^3 40 us (66), 33^3 68 (126), 49^3 99 (203), 65^3 137 (289), 81^3 222 (455),
+// 97^3 296 (744), 113^3 399 (1244).  One group of threads for all rows of a
+// half-sweep: 81^3 300, 49^3 150.
 //
 // Why a neighbour stays within wlag rows: half-sweep q of the lower plane can
 // run row J only after this plane's half-sweep q-1 ran row J+1, which is at
@@ -963,22 +967,29 @@ int launch_gs27_planes(cudaStream_t s, Grid g, Op op, const double* cc, const do
 // The counters hold the launch count of each plane (the tag is that plus
 // one).  A wait that runs out is counted in *err like the counter kernel's.
 // ---------------------------------------------------------------------------
-constexpr int kMailWorkers = 256;   // at most: four half-sweeps of two warps
-constexpr int kMailCouriers = 96;   // and one warp that loads
-constexpr int kMailHelpers = kMailCouriers + 32;
+constexpr int kMailCouriers = 64;
+constexpr int kMailHelpers = kMailCouriers + 64;  // and two warps that load
 constexpr int kMailHalfMax = 4;     // half-sweeps per launch
-constexpr int kMailLagMax = 6;      // rows between successive half-sweeps, at most
-// rows of x a CTA keeps of each plane: from the last half-sweep's lowest to
-// the first one's highest, and some loaded ahead
-constexpr int kMailRows = 26;
-constexpr int kMailInRows = 8;      // rows of the inbox
-static_assert(kMailRows >= kMailLagMax * (kMailHalfMax - 1) + 5 &&
-              kMailInRows >= kMailLagMax + 2, "rings of k_gs27_mail");
 constexpr int kMailPutMax = 2 * kMailHalfMax - 1;  // half-sweeps the inbox holds: 4 of the lower
                                                    // plane, 3 of the upper
 constexpr int kPackPairs = 14;      // pairs of doubles per point of k_gs27_pack
-// stages of packed coefficients per half-sweep, as shared memory allows
+// threads of one group (the rows of one parity of a half-sweep)
+__host__ __device__ constexpr int mail_width(int hp) { return (hp + 31) / 32 * 32; }
+// Per row width: stages of packed coefficients per half-sweep, and rows between
+// successive half-sweeps at most -- the more, the less a plane's progress hangs
+// on its neighbours' (81^3: 294 us at 6 rows, 242 at 8; 49^3: 140, 113, 100 at
+// 12), as many as shared memory holds.
 __host__ __device__ constexpr int mail_stages(int hp) { return hp <= 40 ? 3 : 2; }
+__host__ __device__ constexpr int mail_lag(int hp) {
+  return hp <= 32 ? 14 : (hp <= 40 ? 11 : (hp <= 48 ? 10 : 8));
+}
+// rows of x a CTA keeps of each plane: from the last half-sweep's lowest to
+// the first one's highest, and some loaded ahead
+__host__ __device__ constexpr int mail_xrows(int hp) {
+  return mail_lag(hp) * (kMailHalfMax - 1) + 6;
+}
+// rows of the inbox: a neighbour is less than that far ahead
+__host__ __device__ constexpr int mail_irows(int hp) { return mail_lag(hp) - 1; }
 
 __device__ __forceinline__ void mail_put(unsigned long long* p, double v, unsigned tag) {
   const unsigned long long b = (unsigned long long)__double_as_longlong(v);
@@ -1017,7 +1028,8 @@ size_t gs27_pack_doubles(Grid g) {
 static size_t mail_smem(Grid g) {
   const size_t hp = pack_hr(g);
   return mail_stages((int)hp) * kMailHalfMax * kPackPairs * hp * 16 +
-         3 * kMailRows * 2 * (hp + 2) * sizeof(double) + kMailPutMax * kMailInRows * hp * 16;
+         3 * mail_xrows((int)hp) * 2 * (hp + 1) * sizeof(double) +
+         kMailPutMax * mail_irows((int)hp) * hp * 16;
 }
 
 // The packed coefficients of a 27-point level; coef 0: only the pair (D, 1/D),
@@ -1066,12 +1078,12 @@ void launch_gs27_pack(cudaStream_t s, Grid g, Op op, const double* cc, double* p
                                                  coef);
 }
 
-// What one step leaves for the next step's update of a point: the sums and
-// products that do not wait for that step's mail.
+// The sums and products of one point's update that do not wait for its late
+// neighbours.
 struct Ready27 {
-  double o, u, d0, d2, d3, d4, d5, d6, d7, d8;  // partial tO, tU, products of tD
-  double a1, a6, a7;                            // couplings of the late neighbours
-  double f, diag, rdiag;
+  double o, u, d0, d2, d5, d6, d7, d8;  // partial tO, tU, products of tD
+  double a1, a3, a4, a6, a7;            // couplings of the late neighbours
+  double diag, rdiag;
 };
 
 // a cluster's shared memory: the address of this CTA's `p` in CTA `rank`
@@ -1111,14 +1123,15 @@ __device__ __forceinline__ bool mbar_done(unsigned bar, unsigned parity) {
 
 // HP: pack_hr of the level.  A single warp per scheduler runs most of a step,
 // so its length is its instruction count: strides are compile-time constants,
-// rows and slots are reached by increments, and the two colour offsets of a
-// row have a copy of the step each (a thread alternates between them).
+// rows and slots are reached by increments, and the two groups of a half-sweep,
+// which differ in the columns of their points, have a copy of the code each.
 template <int HP>
-__global__ void __launch_bounds__(kMailWorkers + kMailHelpers, 1)
+__global__ void __launch_bounds__(2 * kMailHalfMax * mail_width(HP) + kMailHelpers, 1)
     k_gs27_mail(Grid g, const double2* __restrict__ pk, const double* __restrict__ fc, double* x,
                 int x_zero, int nhalf, int first_parity, unsigned* counters, int* err, int wlag,
                 unsigned long long* mail) {
-  constexpr unsigned RUN = HP + 2;              // values of one column parity of a row (even)
+  constexpr int kMailRows = mail_xrows(HP), kMailInRows = mail_irows(HP);
+  constexpr unsigned RUN = HP + 1;              // values of one column parity of a row
   constexpr unsigned RL = 2 * RUN;              // a row: its even-i values, then its odd-i ones
   constexpr unsigned PS = RL * kMailRows;       // a plane
   constexpr unsigned IROW = 2 * HP;             // words of an inbox row
@@ -1132,9 +1145,10 @@ __global__ void __launch_bounds__(kMailWorkers + kMailHelpers, 1)
   unsigned long long* inbox = reinterpret_cast<unsigned long long*>(ring + 3 * PS);
   __shared__ unsigned long long full[kMailHalfMax][NS];
   __shared__ unsigned tag_sh;
-  // the last row of x loaded; per half-sweep the step all its threads have
-  // entered (row before it updated, products of its row made)
-  __shared__ volatile int rows_sh, prog_sh[kMailHalfMax];
+  // the last row of x loaded; per half-sweep and group the last row whose upper
+  // mail is taken, whose products are made, that is updated
+  __shared__ volatile int rows_sh, up_sh[kMailHalfMax][2], prod_sh[kMailHalfMax][2],
+      done_sh[kMailHalfMax][2];
   __shared__ volatile int failed_sh;
   cg::cluster_group cl = cg::this_cluster();
   const int rank = (int)cl.block_rank(), clsize = (int)cl.num_blocks();
@@ -1148,7 +1162,8 @@ __global__ void __launch_bounds__(kMailWorkers + kMailHelpers, 1)
     tag_sh = has_plane ? counters[c] + 1u : 0u;
     rows_sh = 3;
     failed_sh = 0;
-    for (int q = 0; q < kMailHalfMax; q++) prog_sh[q] = -2;
+    for (int q = 0; q < kMailHalfMax; q++)
+      for (int h = 0; h < 2; h++) up_sh[q][h] = prod_sh[q][h] = done_sh[q][h] = -1;
     for (int q = 0; q < kMailHalfMax; q++)
       for (int t = 0; t < NS; t++)
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(
@@ -1183,7 +1198,7 @@ __global__ void __launch_bounds__(kMailWorkers + kMailHelpers, 1)
   asm volatile("cp.async.wait_all;" ::: "memory");
   cl.sync();  // every inbox of the cluster is clear before anyone writes one
   const unsigned tag = tag_sh;
-  const unsigned itag0 = tag * 64u + 1u;  // inbox tag of lap 0 (at most 127 / 8 laps)
+  const unsigned itag0 = tag * 64u + 1u;  // inbox tag of lap 0 (at most 113 / 7 laps)
   volatile int* verr = err;
   // a wait's bound: false once it ran out, here or elsewhere
   auto keep_waiting = [&](unsigned long long& t0) -> bool {
@@ -1201,50 +1216,20 @@ __global__ void __launch_bounds__(kMailWorkers + kMailHelpers, 1)
 
   if (!has_plane) {
     // only the barriers
-  } else if ((int)threadIdx.x >= nwork + kMailCouriers) {
-    // ---- the loading warp: rows of x, and by lane q the coefficients of
-    // half-sweep q as the workers free their stages (bulk copies: they take no
-    // part of the load pipe that the workers' critical loads wait for)
+  } else if ((int)threadIdx.x >= nwork + kMailCouriers + 32) {
+    // ---- the warp that loads rows of x
     const int lane = threadIdx.x & 31;
-    const int q = lane < nhalf ? lane : nhalf - 1;
-    int next = lane < nhalf ? 1 : ny;  // the next row of coefficients this lane copies
-    int xnext = 4, last = 0;
     unsigned long long t0 = 0;
-    for (int spins = 1;; spins++) {
-      const int lim = min(ny - 2, max(0, prog_sh[q]) + NS);
-      for (; next <= lim; next++) {
-        const int st = (next - 1) % NS;
-        const unsigned bar = (unsigned)__cvta_generic_to_shared(&full[q][st]);
-        const double2* src =
-            pk + (((size_t)(k - 1) * (ny - 2) + (next - 1)) * 2 + ((first_parity + q) & 1)) * REC;
-        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar),
-                     "r"(REC * 16u)
-                     : "memory");
-        asm volatile(
-            "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, "
-            "[%3];" ::"r"((unsigned)__cvta_generic_to_shared(coef + (q * NS + st) * REC)),
-            "l"(src), "r"(REC * 16u), "r"(bar)
-            : "memory");
-        if (next + 4 <= ny - 2)
-          asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src + 8 * (size_t)REC),
-                       "r"(REC * 16u)
-                       : "memory");
-      }
-      __syncwarp();
+    for (int xnext = 4, spins = 1; xnext < ny; spins++) {
       // a row's slot is free once the last half-sweep's reads are above it
-      const int xlim = min(min(ny - 1, xnext + 3), prog_sh[nhalf - 1] + kMailRows - 2);
-      const int done = __shfl_sync(0xffffffffu, xlim, 0);
-      if (xnext <= done) {
-        for (; xnext <= done; xnext++) load_row(xnext, lane, 32);
+      const int low = min(done_sh[nhalf - 1][0], done_sh[nhalf - 1][1]);
+      const int lim = __shfl_sync(0xffffffffu, min(min(ny - 1, xnext + 3), low + kMailRows - 2), 0);
+      if (xnext <= lim) {
+        for (; xnext <= lim; xnext++) load_row(xnext, lane, 32);
         asm volatile("cp.async.wait_all;" ::: "memory");
         __threadfence_block();
         __syncwarp();
-        if (lane == 0) rows_sh = done;
-      }
-      if (__all_sync(0xffffffffu, xnext >= ny && next > ny - 2)) break;
-      const int at = xnext + __shfl_sync(0xffffffffu, next, 0);
-      if (at != last) {
-        last = at;
+        if (lane == 0) rows_sh = lim;
         t0 = 0;
       }
       if ((spins & 63) == 0) {
@@ -1253,14 +1238,48 @@ __global__ void __launch_bounds__(kMailWorkers + kMailHelpers, 1)
         if (!__shfl_sync(0xffffffffu, go, 0)) break;
       }
     }
-    // a copy must not outlive the CTA: those the workers did not wait for
-    // (after a failure) are waited for here
-    if (lane < nhalf)
+  } else if ((int)threadIdx.x >= nwork + kMailCouriers) {
+    // ---- the warp that loads coefficients: lane q those of half-sweep q, as the
+    // workers free their stages (bulk copies: they take no part of the load pipe
+    // that the workers' critical loads wait for)
+    const int q = threadIdx.x & 31;
+    if (q < nhalf) {
+      const int par = (first_parity + q) & 1;
+      const double2* src = pk + ((size_t)(k - 1) * (ny - 2) * 2 + par) * REC;
+      unsigned long long t0 = 0;
+      int next = 1;
+      for (int spins = 1; next <= ny - 2; spins++) {
+        // the stage holds row next - NS until its products are made
+        const int old = next - NS;
+        if (old < 1 || prod_sh[q][((1 + old + k) & 1) ^ par] >= old) {
+          const int st = (next - 1) % NS;
+          const unsigned bar = (unsigned)__cvta_generic_to_shared(&full[q][st]);
+          asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar),
+                       "r"(REC * 16u)
+                       : "memory");
+          asm volatile(
+              "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, "
+              "[%3];" ::"r"((unsigned)__cvta_generic_to_shared(coef + (q * NS + st) * REC)),
+              "l"(src), "r"(REC * 16u), "r"(bar)
+              : "memory");
+          if (next + 4 <= ny - 2)
+            asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src + 8 * (size_t)REC),
+                         "r"(REC * 16u)
+                         : "memory");
+          src += 2 * REC;
+          next++;
+          t0 = 0;
+        }
+        if ((spins & 63) == 0 && !keep_waiting(t0)) break;
+      }
+      // a copy must not outlive the CTA: those the workers did not wait for
+      // (after a failure) are waited for here
       for (int r = max(1, next - NS); r < next; r++) {
         const unsigned bar = (unsigned)__cvta_generic_to_shared(&full[q][(r - 1) % NS]);
         for (int n = 0; n < (1 << 20) && !mbar_done(bar, ((r - 1) / NS) & 1); n++) {
         }
       }
+    }
   } else if ((int)threadIdx.x >= nwork) {
     // ---- couriers: the foreign neighbour's global slots into the inbox
     const int side = (rank == 0 && c > 0) ? 0 : ((rank == clsize - 1 && c + 1 < ncta) ? 1 : -1);
@@ -1309,7 +1328,7 @@ __global__ void __launch_bounds__(kMailWorkers + kMailHelpers, 1)
           const unsigned long long it =
               (unsigned long long)(itag0 + (unsigned)row[n] / kMailInRows) << 32;
           unsigned long long* s = inbox + (side * kMailHalfMax + q[n]) * IBOX +
-                                  (row[n] & (kMailInRows - 1)) * IROW + 2 * m[n];
+                                  (row[n] % kMailInRows) * IROW + 2 * m[n];
           inbox_put((unsigned)__cvta_generic_to_shared(s), (w[n][d][0] & 0xffffffffull) | it,
                     (w[n][d][1] & 0xffffffffull) | it);
           row[n] = d == 0 ? nrow[n] : valid_from(n, row[n] + 1);
@@ -1319,167 +1338,168 @@ __global__ void __launch_bounds__(kMailWorkers + kMailHelpers, 1)
       if ((spins & 63) == 0 && !keep_waiting(t0)) break;
     }
   } else {
-    // ---- workers: this thread's half-sweep, slot and colour
-    const int width = nwork / nhalf;
-    const int q = threadIdx.x / width, m = threadIdx.x - q * width;
+    // ---- workers: this thread's half-sweep, group and slot
+    constexpr int W = mail_width(HP);
+    const int gid = threadIdx.x / W, q = gid >> 1, m = threadIdx.x - gid * W;
     const int par = (first_parity + q) & 1;
-    // the points of row j are i = 1 + b + 2m, b alternating from row to row;
-    // the last slot of a row with b = 1 is empty.  The lower plane's row j+1
-    // and the upper plane's row j+2 (of the other colour) have the same i.
-    const bool on[2] = {m < hr, m < hr - 1};
+    const int b_of_0 = (((1 + k) & 1) != par) ? 1 : 0;  // the group of row 0
     const bool has_lo = c > 0, has_up = c + 1 < ncta && q > 0;
-    // (lanes beyond the row poll slot 0, without use)
-    const unsigned in_lo =
-        (unsigned)__cvta_generic_to_shared(inbox + q * IBOX + 2 * (m < HP ? m : 0));
-    const unsigned in_up = (unsigned)__cvta_generic_to_shared(
-        inbox + (kMailHalfMax + (q > 0 ? q - 1 : 0)) * IBOX + 2 * (m < HP ? m : 0));
     // where this thread's updates go: the upper plane's inbox, the lower
     // plane's (if a later half-sweep reads them there), the global slot
     const bool to_up = c + 1 < ncta, to_lo = c > 0 && q + 1 < nhalf;
     const bool in_cl_up = to_up && rank + 1 < clsize, in_cl_lo = to_lo && rank > 0;
     const bool to_global = (to_up && !in_cl_up) || (to_lo && !in_cl_lo);
     const bool to_x = q >= nhalf - 2;
-    const unsigned out_up = in_cl_up ? cluster_addr(inbox + q * IBOX + 2 * m, rank + 1) : 0u;
-    const unsigned out_lo =
-        in_cl_lo ? cluster_addr(inbox + (kMailHalfMax + q) * IBOX + 2 * m, rank - 1) : 0u;
-    unsigned long long* own =  // slot of row j, which starts at -1
-        mail + 2 * ((((ptrdiff_t)c * nhalf + q) * (ny - 2) - 2) * hr + m);
-    // row j of x at column 1 + 2m, row j + 2 of f
-    double* xrow = x + ((ptrdiff_t)k * ny - 1) * nx + 1 + 2 * m;
-    const double* frow = fc + (ptrdiff_t)k * ny * nx + 1 + 2 * m;
-    // the stage of row j + 1's coefficients, with the parity of its barrier
-    const double2* cst = coef + q * NS * REC + m;
-    const unsigned bar0 = (unsigned)__cvta_generic_to_shared(&full[q][0]);
-    unsigned stage = 0, parity = 0;
-    // ring offsets of rows j-1, j, j+1 at slot m; inbox rows j, j+1 (byte
-    // offset and tag)
-    auto next_row = [&](unsigned o) -> unsigned {
-      return o + RL >= PS + (unsigned)m ? o + RL - PS : o + RL;
+    auto group_sync = [&]() {
+      if (W == 32) __syncwarp();
+      else asm volatile("bar.sync %0, %1;" ::"r"(1 + gid), "n"(W) : "memory");
     };
-    unsigned om = (kMailRows - 2) * RL + m, o0 = (kMailRows - 1) * RL + m, op = m;  // j = -1
-    unsigned ia = (kMailInRows - 1) * (8u * IROW), ib = 0, ta = itag0 - 1u, tb = itag0;
-    volatile int* prev = &prog_sh[q > 0 ? q - 1 : 0];
-    volatile int* follow = &prog_sh[q + 1 < nhalf ? q + 1 : q];
-    double fnext = 0.0;  // f of row j + 1
-    // f of the row frow is at (B: its colour offset), then on to the next
-    auto fetch = [&](auto bsel, int j) {
+    // The rows of the group whose points are i = 1 + B + 2m (row 0 and row
+    // ny - 1 only take mail and mark progress).
+    auto rows_of = [&](auto bsel) {
       constexpr int B = decltype(bsel)::value;
-      if (on[B] && (unsigned)(j - 1) < (unsigned)(ny - 2)) fnext = __ldg(frow + B);
-      frow += nx;
-    };
-    // step j (row j, colour offset B)
-    auto step = [&](auto bsel, int j, Ready27& R) {
-      constexpr int B = decltype(bsel)::value;
-      constexpr int oc = B == 0 ? RUN : 1, oe = B == 0 ? 1 : RUN + 1;      // row j's columns
-      constexpr int nc = B == 0 ? 1 : RUN, ne = B == 0 ? RUN + 1 : 1;      // row j+1's
-      const unsigned on2 = next_row(op);                                   // row j+2
-      const unsigned ic = ib + 8u * IROW == 8u * IBOX ? 0u : ib + 8u * IROW;
-      const unsigned tc = ic == 0u ? tb + 1u : tb;
-      // what the step waits for: its mail; for its end rows of x, coefficients
-      // and the half-sweep before it three rows ahead; the one after it within
-      // wlag rows.  The loads are issued together.
-      const bool lo = has_lo && on[B] && (unsigned)j < (unsigned)(ny - 2);
-      const bool up = has_up && on[B] && (unsigned)(j + 1) < (unsigned)(ny - 2);
-      const bool prep = (unsigned)j < (unsigned)(ny - 2);
-      const int want = min(j + 2, ny - 1);
-      const int ahead = q > 0 && prep ? min(j + 3, ny - 1) : -2;
-      const int behind = q + 1 < nhalf ? j - wlag : -2;
-      const unsigned bar = bar0 + 8u * stage;
-      unsigned long long w0, w1, v0, v1, t0 = 0;
-      for (int spins = 1;; spins++) {
-        inbox_load(in_lo + ib, w0, w1);
-        inbox_load(in_up + ic, v0, v1);
-        const int rows = rows_sh, pa = *prev, pb = *follow;
-        const bool there = mbar_done(bar, parity);
-        if ((!lo || mail_is(w0, w1, tb)) && (!up || mail_is(v0, v1, tc)) && rows >= want &&
-            pa >= ahead && pb >= behind && (there || !prep))
-          break;
-        if ((spins & 255) == 0 && !keep_waiting(t0)) break;
-      }
-      if (lo) ring[op + oc] = __longlong_as_double((long long)((w1 << 32) | (unsigned)w0));
-      if (up)
-        ring[2 * PS + on2 + oc] = __longlong_as_double((long long)((v1 << 32) | (unsigned)v0));
-      // the threads of the half-sweep
-      if (width == 32) __syncwarp();
-      else asm volatile("bar.sync %0, %1;" ::"r"(1 + q), "r"(width) : "memory");
-      if (m == 0) prog_sh[q] = j;
-      if (on[B] && (unsigned)(j - 1) < (unsigned)(ny - 2)) {
-        // the late neighbours, the rest of the sums in the reference's order
-        const double tD = R.d0 + R.a1 * ring[op + oc] + R.d2 + R.d3 + R.d4 + R.d5 + R.d6 + R.d7 +
-                          R.d8;
-        const double tO = R.o + R.a6 * ring[PS + om + oe] + R.a7 * ring[PS + om + oe - 1];
-        const double v = div_by(R.f + (tO + R.u + tD), R.diag, R.rdiag);
-        const unsigned long long bits = (unsigned long long)__double_as_longlong(v);
-        const unsigned long long it = (unsigned long long)ta << 32;
-        const unsigned long long w0 = (bits & 0xffffffffull) | it, w1 = (bits >> 32) | it;
-        if (in_cl_up) inbox_put(out_up + ia, w0, w1);
-        if (in_cl_lo) inbox_put(out_lo + ia, w0, w1);
-        if (to_global) mail_put(own, v, tag);
-        ring[PS + o0 + oc] = v;
-        if (to_x) __stcg(xrow + B, v);
-      }
-      own += 2 * hr;
-      xrow += nx;
-      om = o0;
-      o0 = op;
-      op = on2;
-      ia = ib;
-      ib = ic;
-      ta = tb;
-      tb = tc;
-      // the next row's early products, from its coefficients
-      if (prep) {
-        if (on[1 - B]) {
-          const double2* cp = cst + stage * REC;
-          const double* rm = ring + om;
-          const double* r0 = ring + o0;
-          const double* rp = ring + op;
-          auto K = [&](int t) -> double2 { return cp[t * HP]; };
-          const double2 k0 = K(0), k1 = K(1), k2 = K(2), k3 = K(3), k4 = K(4), k5 = K(5),
-                        k6 = K(6), k7 = K(7), k8 = K(8), k9 = K(9), k10 = K(10), k11 = K(11),
-                        k12 = K(12), k13 = K(13);
-          R.o = +k0.x * rp[PS + nc] + k0.y * rm[PS + nc] + k1.x * r0[PS + ne] +
-                k1.y * r0[PS + ne - 1] + k2.x * rp[PS + ne] + k2.y * rp[PS + ne - 1];
-          R.u = +k4.x * r0[2 * PS + nc] + k4.y * rp[2 * PS + nc] + k5.x * rm[2 * PS + nc] +
-                k5.y * r0[2 * PS + ne] + k6.x * r0[2 * PS + ne - 1] + k6.y * rp[2 * PS + ne] +
-                k7.x * rp[2 * PS + ne - 1] + k7.y * rm[2 * PS + ne] + k8.x * rm[2 * PS + ne - 1];
-          R.d0 = k8.y * r0[nc];
-          R.d2 = k9.y * rm[nc];
-          R.d3 = k10.x * r0[ne];
-          R.d4 = k10.y * r0[ne - 1];
-          R.d5 = k11.x * rp[ne];
-          R.d6 = k11.y * rp[ne - 1];
-          R.d7 = k12.x * rm[ne];
-          R.d8 = k12.y * rm[ne - 1];
-          R.a1 = k9.x;
-          R.a6 = k3.x;
-          R.a7 = k3.y;
-          R.f = fnext;
-          R.diag = k13.x;
-          R.rdiag = k13.y;
+      // the row's points; those of the lower plane's row j+1 are the same, those
+      // of the upper plane's row j+1 (of the other colour) the other group's
+      constexpr unsigned oc = B == 0 ? RUN : 1, oe = B == 0 ? 1 : RUN + 1;
+      const bool on = B == 0 ? m < hr : m < hr - 1, on_up = B == 0 ? m < hr - 1 : m < hr;
+      int j = b_of_0 == B ? 0 : 1;
+      unsigned st = j == 0 ? 1u : 0u, parity = 0;  // stage of the next row's coefficients
+      // ring offsets of rows j-1, j, j+1 at slot m; inbox rows j, j+1 (byte
+      // offset and tag)
+      auto next_row = [&](unsigned o) -> unsigned {
+        return o + RL >= PS + (unsigned)m ? o + RL - PS : o + RL;
+      };
+      unsigned om = (j == 0 ? (kMailRows - 1) * RL : 0u) + m, o0 = j * RL + m, op = o0 + RL;
+      unsigned ia = (unsigned)j * (8u * IROW), ib = ia + 8u * IROW, ta = itag0, tb = itag0;
+      const unsigned slot = 2u * (m < HP ? m : 0);  // lanes beyond the row poll slot 0, unused
+      const unsigned in_lo = (unsigned)__cvta_generic_to_shared(inbox + q * IBOX + slot);
+      const unsigned in_up = (unsigned)__cvta_generic_to_shared(
+          inbox + (kMailHalfMax + (q > 0 ? q - 1 : 0)) * IBOX + slot);
+      const unsigned out_up = in_cl_up ? cluster_addr(inbox + q * IBOX + slot, rank + 1) : 0u;
+      const unsigned out_lo =
+          in_cl_lo ? cluster_addr(inbox + (kMailHalfMax + q) * IBOX + slot, rank - 1) : 0u;
+      unsigned long long* own =  // global slot of row j
+          mail + 2 * ((((ptrdiff_t)c * nhalf + q) * (ny - 2) + j - 1) * hr + m);
+      double* xrow = x + ((size_t)k * ny + j) * nx + 1 + B + 2 * m;
+      const double* frow = fc + ((size_t)k * ny + j) * nx + 1 + B + 2 * m;
+      const double2* cst = coef + q * NS * REC + m;
+      const unsigned bar0 = (unsigned)__cvta_generic_to_shared(&full[q][0]);
+      // progress this group waits for: the other group, row j+1 of the half-sweep
+      // before (its group B), row j-wlag of the one after
+      const volatile int* other_up = &up_sh[q][1 - B];
+      const volatile int* other_done = &done_sh[q][1 - B];
+      const volatile int* before = &done_sh[q > 0 ? q - 1 : 0][B];
+      const volatile int* after = &done_sh[q + 1 < nhalf ? q + 1 : q][(wlag & 1) ? B : 1 - B];
+      double f = j == 0 || !on ? 0.0 : __ldg(frow);  // of row j
+      for (; j <= ny - 1; j += 2) {
+        const bool inner = (unsigned)(j - 1) < (unsigned)(ny - 2);
+        const bool mailed = j < ny - 2;  // row j + 1 is one of the neighbours' rows too
+        const bool up = has_up && on_up && mailed, lo = has_lo && on && mailed;
+        const unsigned bar = bar0 + 8u * st;
+        unsigned long long w0, w1, t0 = 0;
+        {
+          const int want_rows = min(j + 1, ny - 1);
+          const int want_before = q > 0 && inner ? j + 1 : -1;
+          const int want_after = q + 1 < nhalf ? j - wlag : -1;
+          for (int spins = 1;; spins++) {
+            inbox_load(in_up + ib, w0, w1);
+            const int r = rows_sh, u = *other_up, p = *before, n = *after;
+            const bool there = mbar_done(bar, parity);
+            if ((!up || mail_is(w0, w1, tb)) && r >= want_rows && u >= j - 1 && p >= want_before &&
+                n >= want_after && (there || !inner))
+              break;
+            if ((spins & 255) == 0 && !keep_waiting(t0)) break;
+          }
+          if (up)
+            ring[2 * PS + op + (B == 0 ? 1u : RUN)] =
+                __longlong_as_double((long long)((w1 << 32) | (unsigned)w0));
         }
-        stage++;
-        if (stage == NS) {
-          stage = 0;
-          parity ^= 1u;
+        group_sync();
+        if (m == 0) up_sh[q][B] = j;
+        Ready27 R;
+        if (inner) {
+          // the products, and the sums before them, that need no late neighbour
+          if (on) {
+            const double2* cp = cst + st * REC;
+            const double* rm = ring + om;
+            const double* r0 = ring + o0;
+            const double* rp = ring + op;
+            auto K = [&](int t) -> double2 { return cp[t * HP]; };
+            const double2 k0 = K(0), k1 = K(1), k2 = K(2), k3 = K(3), k4 = K(4), k5 = K(5),
+                          k6 = K(6), k7 = K(7), k8 = K(8), k9 = K(9), k10 = K(10), k11 = K(11),
+                          k12 = K(12), k13 = K(13);
+            R.o = +k0.x * rp[PS + oc] + k0.y * rm[PS + oc] + k1.x * r0[PS + oe] +
+                  k1.y * r0[PS + oe - 1] + k2.x * rp[PS + oe] + k2.y * rp[PS + oe - 1];
+            R.u = +k4.x * r0[2 * PS + oc] + k4.y * rp[2 * PS + oc] + k5.x * rm[2 * PS + oc] +
+                  k5.y * r0[2 * PS + oe] + k6.x * r0[2 * PS + oe - 1] + k6.y * rp[2 * PS + oe] +
+                  k7.x * rp[2 * PS + oe - 1] + k7.y * rm[2 * PS + oe] +
+                  k8.x * rm[2 * PS + oe - 1];
+            R.d0 = k8.y * r0[oc];
+            R.d2 = k9.y * rm[oc];
+            R.d5 = k11.x * rp[oe];
+            R.d6 = k11.y * rp[oe - 1];
+            R.d7 = k12.x * rm[oe];
+            R.d8 = k12.y * rm[oe - 1];
+            R.a1 = k9.x;
+            R.a3 = k10.x;
+            R.a4 = k10.y;
+            R.a6 = k3.x;
+            R.a7 = k3.y;
+            R.diag = k13.x;
+            R.rdiag = k13.y;
+          }
+          group_sync();
+          if (m == 0) prod_sh[q][B] = j;
+          st += 2;
+          if (st >= NS) {
+            st -= NS;
+            parity ^= 1u;
+          }
         }
+        // the late neighbours: the lower plane's row j + 1 by mail, its row j
+        // and this plane's row j - 1 from the other group's step
+        t0 = 0;
+        for (int spins = 1;; spins++) {
+          inbox_load(in_lo + ib, w0, w1);
+          const int d = *other_done;
+          if ((!lo || mail_is(w0, w1, tb)) && d >= j - 1) break;
+          if ((spins & 255) == 0 && !keep_waiting(t0)) break;
+        }
+        const double mail1 = __longlong_as_double((long long)((w1 << 32) | (unsigned)w0));
+        if (inner && on) {
+          const double d1 = lo ? mail1 : ring[op + oc];
+          const double tD = R.d0 + R.a1 * d1 + R.d2 + R.a3 * ring[o0 + oe] +
+                            R.a4 * ring[o0 + oe - 1] + R.d5 + R.d6 + R.d7 + R.d8;
+          const double tO = R.o + R.a6 * ring[PS + om + oe] + R.a7 * ring[PS + om + oe - 1];
+          const double v = div_by(f + (tO + R.u + tD), R.diag, R.rdiag);
+          const unsigned long long bits = (unsigned long long)__double_as_longlong(v);
+          const unsigned long long it = (unsigned long long)ta << 32;
+          const unsigned long long o_lo = (bits & 0xffffffffull) | it, o_hi = (bits >> 32) | it;
+          if (in_cl_up) inbox_put(out_up + ia, o_lo, o_hi);
+          if (in_cl_lo) inbox_put(out_lo + ia, o_lo, o_hi);
+          ring[PS + o0 + oc] = v;
+          if (to_global) mail_put(own, v, tag);
+          if (to_x) __stcg(xrow, v);
+        }
+        if (lo) ring[op + oc] = mail1;
+        group_sync();
+        if (m == 0) done_sh[q][B] = j;
+        // on to row j + 2
+        own += 4 * hr;
+        xrow += 2 * nx;
+        frow += 2 * nx;
+        if (on && j + 2 <= ny - 2) f = __ldg(frow);
+        om = op;
+        o0 = next_row(op);
+        op = next_row(o0);
+        ia = ia + 16u * IROW >= 8u * IBOX ? ia + 16u * IROW - 8u * IBOX : ia + 16u * IROW;
+        ib = ib + 16u * IROW >= 8u * IBOX ? ib + 16u * IROW - 8u * IBOX : ib + 16u * IROW;
+        ta = itag0 + (unsigned)(j + 2) / kMailInRows;
+        tb = itag0 + (unsigned)(j + 3) / kMailInRows;
       }
-      fetch(bsel, j + 2);
     };
-
-    // row -1 has colour offset b0; the loop starts with an offset-0 step,
-    // skipped (j = -2) where row -1 has offset 1.  The last step only says
-    // that row ny - 2 is updated.
-    const std::integral_constant<int, 0> B0{};
-    const std::integral_constant<int, 1> B1{};
-    const int b0 = ((k & 1) != par) ? 1 : 0;
-    Ready27 R;
-    if (b0) fetch(B0, 0);
-    else fetch(B1, 0);
-    for (int j = -1 - b0; j <= ny - 1; j += 2) {
-      if (j >= -1) step(B0, j, R);
-      if (j + 1 <= ny - 1) step(B1, j + 1, R);
-    }
+    if (gid & 1) rows_of(std::integral_constant<int, 1>());
+    else rows_of(std::integral_constant<int, 0>());
     if (threadIdx.x == 0) counters[c] = tag;
   }
   cl.sync();  // no CTA exits while a neighbour may write its inbox
@@ -1511,7 +1531,7 @@ static MailPlan mail_plan(Grid g, int nhalf) {
   MailPlan p;
   const int planes = g.nz - 2;
   const MailKernel kernel = mail_kernel(g);
-  p.threads = nhalf * ((mail_hr(g) + 31) / 32 * 32) + kMailHelpers;
+  p.threads = 2 * nhalf * mail_width(pack_hr(g)) + kMailHelpers;
   p.smem = mail_smem(g);
   int dev = 0, lim = 0;
   cudaGetDevice(&dev);
@@ -1557,7 +1577,7 @@ int launch_gs27_mail(cudaStream_t s, Grid g, const double* pack, const double* f
   if (!mail || !pack || nhalf < 3 || nhalf > kMailHalfMax) return 0;
   const MailPlan p = mail_plan(g, nhalf);
   if (!p.kernel) return 0;
-  wlag = std::min(std::max(wlag, 4), kMailLagMax);
+  wlag = wlag < 6 ? std::max(wlag, 4) : mail_lag(pack_hr(g));
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((g.nz - 2 + p.cluster - 1) / p.cluster * p.cluster, 1, 1);
   cfg.blockDim = dim3(p.threads, 1, 1);

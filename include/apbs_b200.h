@@ -222,9 +222,10 @@ int pmgb_solve_molecule(const pmgb_params *params, int precision, int natoms,
                                           sweeps), K > 0 = Jacobi-preconditioned Chebyshev of
                                           degree K (rounded up to even) */
 #define PMGB_TUNE_GS27_LAG 1          /* plane-parallel GS27: wavefronts between successive
-                                          half-sweeps (>= 4, default 6; the mailbox kernel
-                                          takes at most 6); a larger lag lets a plane run
-                                          ahead of the plane above it */
+                                          half-sweeps (>= 4, default 6; from 6 on the mailbox
+                                          kernel takes as many as its shared memory holds);
+                                          a larger lag lets a plane run ahead of the plane
+                                          above it */
 /* key 3 is not used */
 #define PMGB_TUNE_GS27_CLUSTER 2       /* CTAs per cluster of the ordered GS27 on levels with
                                           >= 60 interior points per axis (0 = device max) */
