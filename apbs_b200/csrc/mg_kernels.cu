@@ -8,6 +8,7 @@
 #include <cooperative_groups.h>
 
 #include <algorithm>
+#include <mutex>
 #include <type_traits>
 
 #include "gs7_rb.cuh"
@@ -1520,6 +1521,51 @@ static MailKernel mail_kernel(Grid g) {
   }
 }
 
+// The clusters of 16, 8, 4 and 2 CTAs of one kernel instance that a device holds
+// at once; asked for once per device and instance, as the queries take
+// milliseconds.
+struct MailDevice {
+  std::once_flag once;
+  int clusters[4] = {0, 0, 0, 0};
+};
+static const int* mail_clusters(MailKernel kernel, int hp, int threads, size_t smem) {
+  static MailDevice table[16][8];
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 16) return nullptr;
+  MailDevice& d = table[dev][hp / 8];
+  std::call_once(d.once, [&] {
+    int lim = 0;
+    cudaDeviceGetAttribute(&lim, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    if (smem + 1024 > (size_t)lim ||
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
+            cudaSuccess ||
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) !=
+            cudaSuccess) {
+      cudaGetLastError();
+      return;
+    }
+    for (int t = 0; t < 4; t++) {
+      const int n = 16 >> t;
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3(n, 1, 1);
+      cfg.blockDim = dim3(threads, 1, 1);
+      cfg.dynamicSmemBytes = smem;
+      cudaLaunchAttribute at[1];
+      at[0].id = cudaLaunchAttributeClusterDimension;
+      at[0].val.clusterDim.x = n;
+      at[0].val.clusterDim.y = 1;
+      at[0].val.clusterDim.z = 1;
+      cfg.attrs = at;
+      cfg.numAttrs = 1;
+      if (cudaOccupancyMaxActiveClusters(&d.clusters[t], kernel, &cfg) != cudaSuccess) {
+        d.clusters[t] = 0;
+        cudaGetLastError();
+      }
+    }
+  });
+  return d.clusters;
+}
+
 // The launch of a level: the largest cluster that the device can hold all the
 // planes with at once (fewest hand-overs through global memory).
 struct MailPlan {
@@ -1531,39 +1577,15 @@ static MailPlan mail_plan(Grid g, int nhalf) {
   MailPlan p;
   const int planes = g.nz - 2;
   const MailKernel kernel = mail_kernel(g);
+  if (!kernel || planes < 2 || planes > kWavePlanesMax || nhalf != kMailHalfMax) return p;
   p.threads = 2 * nhalf * mail_width(pack_hr(g)) + kMailHelpers;
   p.smem = mail_smem(g);
-  int dev = 0, lim = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&lim, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-  if (!kernel || planes < 2 || planes > kWavePlanesMax || p.smem + 1024 > (size_t)lim) return p;
-  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem) !=
-          cudaSuccess ||
-      cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) !=
-          cudaSuccess) {
-    cudaGetLastError();
-    return p;
-  }
-  for (int n = 16; n >= 2 && !p.kernel; n /= 2) {
-    if (n > 2 && n / 2 >= planes) continue;
-    const int clusters = (planes + n - 1) / n;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(clusters * n, 1, 1);
-    cfg.blockDim = dim3(p.threads, 1, 1);
-    cfg.dynamicSmemBytes = p.smem;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = n;
-    at[0].val.clusterDim.y = 1;
-    at[0].val.clusterDim.z = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    int fit = 0;
-    if (cudaOccupancyMaxActiveClusters(&fit, kernel, &cfg) == cudaSuccess && fit >= clusters) {
-      p.kernel = kernel;
-      p.cluster = n;
-    }
-    cudaGetLastError();
+  const int* fit = mail_clusters(kernel, pack_hr(g), p.threads, p.smem);
+  for (int t = 0; fit && t < 4 && !p.kernel; t++) {
+    const int n = 16 >> t;
+    if ((n > 2 && n / 2 >= planes) || (planes + n - 1) / n > fit[t]) continue;
+    p.kernel = kernel;
+    p.cluster = n;
   }
   return p;
 }
@@ -1574,7 +1596,7 @@ int launch_gs27_mail(cudaStream_t s, Grid g, const double* pack, const double* f
                      int x_zero, int nsweep, int first_parity, unsigned* counters, int* err,
                      int wlag, unsigned long long* mail) {
   const int nhalf = 2 * nsweep;
-  if (!mail || !pack || nhalf < 3 || nhalf > kMailHalfMax) return 0;
+  if (!mail || !pack) return 0;
   const MailPlan p = mail_plan(g, nhalf);
   if (!p.kernel) return 0;
   wlag = wlag < 6 ? std::max(wlag, 4) : mail_lag(pack_hr(g));

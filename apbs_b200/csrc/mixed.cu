@@ -2043,6 +2043,13 @@ int mixed_time_tail(pmgb_solver* s, double* bytes) {
   return 1;
 }
 
+void launch_band_restencil(cudaStream_t st, Grid g, Op op, double* const* b, int* wrap) {
+  OpW w;
+  for (int c = 0; c < 14; c++) w.c[c] = b[c];
+  const size_t nint = (size_t)(g.nx - 2) * (g.ny - 2) * (g.nz - 2);
+  k_band_restencil<<<blocks_for(nint), kThreads, 0, st>>>(g, op, w, wrap);
+}
+
 // FP64 path, LPBE: prepare the exact coarse solve of the FP64 coarsest level
 // (FP32 Galerkin levels below it and the dense inverse at the bottom).
 // Returns 1 when it is available, 0 when the band solve must be used.
@@ -2065,14 +2072,9 @@ int coarse_exact_prepare(pmgb_solver* s) {
   cudaStream_t st = s->stream;
   MLevel& L = m->lev[lo];
   const Grid g = L.g;
-  const int nint = (g.nx - 2) * (g.ny - 2) * (g.nz - 2);
-  OpW b;
-  for (int c = 0; c < 14; c++) {
-    b.c[c] = L.op64[c];
-    CKM(cudaMemsetAsync(b.c[c], 0, g.n() * sizeof(double), st));
-  }
+  for (int c = 0; c < 14; c++) CKM(cudaMemsetAsync(L.op64[c], 0, g.n() * sizeof(double), st));
   CKM(cudaMemsetAsync(m->d_flag, 0, sizeof(int), st));
-  k_band_restencil<<<blocks_for(nint), kThreads, 0, st>>>(g, s->lev[lo].ops(), b, m->d_flag);
+  launch_band_restencil(st, g, s->lev[lo].ops(), L.op64, m->d_flag);
   note_launches(1);
   int wrap = 0;
   CKM(cudaMemcpyAsync(&wrap, m->d_flag, sizeof(int), cudaMemcpyDeviceToHost, st));

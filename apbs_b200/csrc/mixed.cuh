@@ -22,6 +22,9 @@ int mixed_time_tail(pmgb_solver* s, double* bytes);
 // FP64 path, LPBE: exact-to-round-off solve of the FP64 coarsest level
 // (FP64 refinement over FP32 V-cycles of extra Galerkin levels).
 int coarse_exact_prepare(pmgb_solver* s);
+// The reference's coarsest band matrix as a 27-point operator b (zeroed arrays);
+// *wrap is set where it has an entry that is no grid neighbour's.
+void launch_band_restencil(cudaStream_t st, Grid g, Op op, double* const* b, int* wrap);
 // operator build of solver.cu (Galerkin hierarchy, coarsest factor)
 int solver_build(pmgb_solver* s);
 int launch_coarse_exact(pmgb_solver* s, cudaStream_t st, const double* cc, const double* b,

@@ -19,6 +19,7 @@
 #include <vector>
 
 #include "apbs_b200.h"
+#include "coarse_direct.cuh"
 #include "fill_kernels.cuh"
 #include "mg_kernels.cuh"
 #include "mixed.cuh"
@@ -530,7 +531,13 @@ extern "C" size_t pmgb_footprint(const pmgb_params* params, int precision, int n
   // FP32 hierarchy from level lo, plus Galerkin levels down to <= 512 unknowns
   const int lo = (precision == PMGB_MIXED) ? 0 : nlev - 1;
   const size_t nc_int = (size_t)(gx[nlev - 1] - 2) * (gy[nlev - 1] - 2) * (gz[nlev - 1] - 2);
-  const bool fp32 = (precision == PMGB_MIXED) || (!p.nonlin && nc_int > 512);
+  // the coarsest level's factors where its planes fit, else the FP32 levels of
+  // the refinement
+  const size_t planes = (precision != PMGB_MIXED && !p.nonlin && nc_int > 512)
+                            ? direct_bytes(Grid{gx[nlev - 1], gy[nlev - 1], gz[nlev - 1]})
+                            : 0;
+  bytes += planes;
+  const bool fp32 = (precision == PMGB_MIXED) || (!p.nonlin && nc_int > 512 && planes == 0);
   if (fp32) {
     for (int l = lo; l < nlev; l++)
       bytes += (size_t)((l == 0 ? 4 : 14) + 3) * nl[l] * sizeof(float);
@@ -546,7 +553,7 @@ extern "C" size_t pmgb_footprint(const pmgb_params* params, int precision, int n
       nint = (size_t)(cx - 2) * (cy - 2) * (cz - 2);
     }
     bytes += 2 * nl[lo] * sizeof(float) + nint * nint * sizeof(double);
-  } else if (!p.nonlin) {
+  } else if (!p.nonlin && planes == 0) {
     const size_t ex = gx[nlev - 1] - 2, exy = ex * (gy[nlev - 1] - 2);
     bytes += ((exy + ex + 2) * nc_int + nc_int) * sizeof(double);
   }
@@ -563,6 +570,7 @@ extern "C" void pmgb_destroy(pmgb_solver* s) {
   for (int m = 0; m < 2; m++)
     if (s->vc_exec[m]) cudaGraphExecDestroy(s->vc_exec[m]);
   if (s->mixed) mixed_destroy(s->mixed);
+  direct_destroy(s->direct);
   dfree(s->charge); dfree(s->epsx); dfree(s->epsy); dfree(s->epsz); dfree(s->kappa);
   dfree(s->ccf); dfree(s->gx); dfree(s->gy); dfree(s->gz); dfree(s->xf); dfree(s->yf);
   dfree(s->zf); dfree(s->wx); dfree(s->wy); dfree(s->wz); dfree(s->mom);
@@ -985,12 +993,14 @@ static int build_ops(pmgb_solver* s) {
   // the mixed-precision path solves its own, coarser, level densely instead
   s->mgsolv = (s->p.nonlin || s->precision == PMGB_MIXED) ? 0 : 1;
   if (s->mgsolv == 1) {
-    // a coarsest level above 512 unknowns is solved by exact refinement
-    // instead: the banded factor and its substitutions are sequential
+    // a coarsest level above 512 unknowns is solved by its planes instead, or,
+    // where those do not fit on the device, by exact refinement: the banded
+    // factor and its substitutions are sequential
     const Grid gc = s->lev[s->nlev - 1].g;
-    if ((size_t)(gc.nx - 2) * (gc.ny - 2) * (gc.nz - 2) > 512 && s->tune[4] == 0 &&
-        coarse_exact_prepare(s))
-      s->mgsolv = 2;
+    if ((size_t)(gc.nx - 2) * (gc.ny - 2) * (gc.nz - 2) > 512 && s->tune[4] == 0) {
+      if (direct_prepare(s)) s->mgsolv = 3;
+      else if (coarse_exact_prepare(s)) s->mgsolv = 2;
+    }
   }
   if (s->mgsolv == 1) {
     Level& C = s->lev[s->nlev - 1];
@@ -1124,6 +1134,9 @@ static int vcycle_body(pmgb_solver* s, int newton) {
     Level& C = s->lev[nlev - 1];
     if (s->mgsolv == 1) {
       launch_band_solve(st, C.g, s->band, s->bn, s->bm, s->blda, C.w0, X(nlev - 1));
+      k++;
+    } else if (s->mgsolv == 3) {
+      if (!launch_direct_solve(s, st, C.w0, X(nlev - 1))) return 0;
       k++;
     } else if (s->mgsolv == 2) {
       if (!launch_coarse_exact(s, st, CC(nlev - 1), C.w0, X(nlev - 1))) return 0;
@@ -1402,7 +1415,7 @@ extern "C" int pmgb_solve(pmgb_solver* s) {
   CK(cudaEventRecord(s->ev[2], st));
   if (!s->built && !build_ops(s)) return 0;
   CK(cudaEventRecord(s->ev[3], st));
-  s->st.coarse_method = (s->precision == PMGB_MIXED) ? 2 : (s->mgsolv == 2 ? 3 : s->mgsolv);
+  s->st.coarse_method = (s->precision == PMGB_MIXED) ? 2 : (s->mgsolv >= 2 ? 3 : s->mgsolv);
   const double errtol = (s->p.etol > 0.0) ? s->p.etol : 1.0e-6;
   // Vpmgp itmax (vpmgp.c:131): V-cycles (LPBE) or Newton steps (NPBE)
   const int itmax = (s->p.itmax > 0) ? s->p.itmax : 200;
@@ -1724,6 +1737,7 @@ extern "C" int pmgb_solver_set_tuning(pmgb_solver* s, int key, int value) {
     s->built = 0;
     s->solved = 0;
   }
+  if (s->direct) s->built = s->solved = 0;  // the coarsest solve is chosen again
   return 1;
 }
 

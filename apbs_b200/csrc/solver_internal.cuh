@@ -8,6 +8,7 @@
 
 namespace pmgb {
 struct MixedState;
+struct DirectState;
 void note_launches(long long n);
 }  // namespace pmgb
 
@@ -166,5 +167,6 @@ struct pmgb_solver {
   long long vc_kernels[2];
   int vc_mgsolv[2];  // coarsest-solve kind each graph was captured with
   pmgb::MixedState* mixed;
+  pmgb::DirectState* direct;  // factors of the FP64 coarsest level (LPBE)
 };
 
