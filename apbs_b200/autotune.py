@@ -48,7 +48,7 @@ CANDIDATES = {
     },
     MIXED: {
         TUNE_MIXED_CHEBYSHEV: [2, 0, 4],
-        TUNE_TAIL_MAX_POINTS: [70000, 20000, 5000],
+        TUNE_TAIL_MAX_POINTS: [20000, 70000, 5000],
         TUNE_MIXED_FINE_SWEEPS: [2, 1, 3, 4],
         TUNE_MIXED_COARSE_SWEEPS: [2, 1, 3],
         TUNE_GS7_COLOUR_PASSES: [0, 2],

@@ -61,6 +61,7 @@ struct OpF {
 // one level of the FP32 hierarchy as seen by the tail kernel
 struct TLev {
   Grid g;
+  unsigned dx, dy;   // ceil(2^32 / (nx - 2)), ceil(2^32 / (ny - 2)): interior_at
   const float* op[14];
   const float* cc;
   float* w0;
@@ -739,13 +740,70 @@ __device__ __forceinline__ float nb27t(const TLev& L, const float* x, size_t id)
   return nb27(o, L.g, x, id);
 }
 
+// q / d by multiplication with div_const(d) = ceil(2^32 / d) (0: d = 1): exact for
+// q < 2^32 / d, which the levels of one cluster are far below.
+inline unsigned div_const(int d) {
+  return d > 1 ? (unsigned)((0x100000000ull + d - 1) / d) : 0u;
+}
+__device__ __forceinline__ int quotient(int q, unsigned c) {
+  return c ? (int)__umulhi((unsigned)q, c) : q;
+}
+// Interior point q of a level as a flat index.
+__device__ __forceinline__ int interior_at(Grid g, unsigned dx, unsigned dy, int q) {
+  const int ex = g.nx - 2, ey = g.ny - 2;
+  const int t = quotient(q, dx), k = quotient(t, dy);
+  return ((k + 1) * g.ny + t - k * ey + 1) * g.nx + q - t * ex + 1;
+}
+
+// A thread's number among those of the cluster, in two orders: CTA by CTA, and
+// warp by warp round the CTAs.  A level with fewer points than threads goes by
+// the second, which spreads it over all the cluster's SMs (17^3: 16 instead of 7;
+// a pass is bounded by what one SM's load pipe takes in).
+struct TailTid {
+  int block, round, n;
+  __device__ __forceinline__ int first(int points) const { return points < n ? round : block; }
+};
+template <int CLUSTER>
+__device__ __forceinline__ TailTid tail_tid() {
+  TailTid t;
+  const int rank = CLUSTER > 1 ? (int)cg::this_cluster().block_rank() : 0;
+  t.block = rank * blockDim.x + threadIdx.x;
+  t.round = (int)(((threadIdx.x >> 5) * CLUSTER + rank) * 32 + (threadIdx.x & 31));
+  t.n = CLUSTER * blockDim.x;
+  return t;
+}
+
+// The thread's points below n, U at a time: value(id) of all of them (id the flat
+// index at(q), or -1: none), then the stores.  The loads of U points
+// are in flight together; a thread's next point would otherwise wait for the
+// stores of the one before, which the compiler must take for its inputs.
+template <int U, class At, class Value, class Store>
+__device__ __forceinline__ void for_points(int n, TailTid tid, At at, Value value, Store store) {
+  const int nthr = tid.n;
+  for (int q0 = tid.first(n); q0 < n; q0 += U * nthr) {
+    int id[U];
+    decltype(value(0)) v[U];
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      const int q = q0 + u * nthr;
+      id[u] = q < n ? at(q) : -1;
+      if (id[u] >= 0) v[u] = value(id[u]);
+    }
+#pragma unroll
+    for (int u = 0; u < U; u++)
+      if (id[u] >= 0) store(id[u], v[u]);
+  }
+}
+
 template <int CLUSTER>
 __device__ __forceinline__ void tail_sync() {
   if (CLUSTER > 1) cg::this_cluster().sync();
   else __syncthreads();
 }
 
-// sum of two values over the cluster, same result in every thread
+// Sum of two values over the cluster, the same result in every thread.  Each CTA
+// stores its partial sums into every CTA's slots ahead of the barrier, so after it
+// they are read locally, in rank order.  slots: [2 phases][CLUSTER][2].
 template <int CLUSTER>
 __device__ void tail_sum2(double& a, double& b, double* sh, double* slots, int& phase) {
   a = warp_sum(a);
@@ -756,36 +814,38 @@ __device__ void tail_sum2(double& a, double& b, double* sh, double* slots, int& 
     sh[2 * wid + 1] = b;
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
+  double* mine = slots + 2 * CLUSTER * phase;
+  if (threadIdx.x < CLUSTER) {
     double sa = 0.0, sb = 0.0;
     for (int w = 0; w < (int)(blockDim.x >> 5); w++) {
       sa += sh[2 * w];
       sb += sh[2 * w + 1];
     }
-    slots[2 * phase] = sa;
-    slots[2 * phase + 1] = sb;
-  }
-  if (CLUSTER > 1) {
-    cg::cluster_group cl = cg::this_cluster();
-    cl.sync();
-    double ta = 0.0, tb = 0.0;
-    for (int rk = 0; rk < CLUSTER; rk++) {
-      double* rs = cl.map_shared_rank(slots, rk);
-      ta += rs[2 * phase];
-      tb += rs[2 * phase + 1];
+    if (CLUSTER > 1) {
+      cg::cluster_group cl = cg::this_cluster();
+      const int rank = (int)cl.block_rank();
+      double* to = cl.map_shared_rank(mine, (int)threadIdx.x) + 2 * rank;
+      to[0] = sa;
+      to[1] = sb;
+    } else {
+      mine[0] = sa;
+      mine[1] = sb;
     }
-    a = ta;
-    b = tb;
-  } else {
-    __syncthreads();
-    a = slots[2 * phase];
-    b = slots[2 * phase + 1];
   }
+  tail_sync<CLUSTER>();
+  double ta = 0.0, tb = 0.0;
+#pragma unroll
+  for (int rk = 0; rk < CLUSTER; rk++) {
+    ta += mine[2 * rk];
+    tb += mine[2 * rk + 1];
+  }
+  a = ta;
+  b = tb;
   phase ^= 1;
 }
 
 template <int CLUSTER>
-__device__ void tail_smooth(const TLev& L, int reverse, int gtid, int nthr, int nsweep) {
+__device__ void tail_smooth(const TLev& L, int reverse, TailTid tid, int nsweep) {
   const Grid g = L.g;
   const int hx = (g.nx - 1) / 2, hy = (g.ny - 1) / 2, hz = (g.nz - 1) / 2;
   const int tot = hx * hy * hz;
@@ -793,7 +853,7 @@ __device__ void tail_smooth(const TLev& L, int reverse, int gtid, int nthr, int 
     for (int c8 = 0; c8 < 8; c8++) {
       const int c = reverse ? 7 - c8 : c8;
       const int pi = c & 1, pj = (c >> 1) & 1, pk = (c >> 2) & 1;
-      for (int t = gtid; t < tot; t += nthr) {
+      for (int t = tid.first(tot); t < tot; t += tid.n) {
         const int mi = t % hx, mj = (t / hx) % hy, mk = t / (hx * hy);
         const int i = (pi ? 1 : 2) + 2 * mi, j = (pj ? 1 : 2) + 2 * mj, k = (pk ? 1 : 2) + 2 * mk;
         if (i > g.nx - 2 || j > g.ny - 2 || k > g.nz - 2) continue;
@@ -804,38 +864,59 @@ __device__ void tail_smooth(const TLev& L, int reverse, int gtid, int nthr, int 
     }
 }
 
-// K Chebyshev steps on level L inside the cluster (K even: the result ends in L.x)
+// Chebyshev steps first .. K-1 on level L inside the cluster (K even: the result
+// ends in L.x)
 template <int CLUSTER>
-__device__ void tail_cheb(const TLev& L, int gtid, int nthr, int K) {
+__device__ void tail_cheb(const TLev& L, TailTid tid, int K, int first) {
   const Grid g = L.g;
+  const unsigned dx = L.dx, dy = L.dy;
   OpF o;
 #pragma unroll
   for (int c = 0; c < 14; c++) o.c[c] = L.op[c];
   o.nop = 14;
-  const int ex = g.nx - 2, ey = g.ny - 2, nint = ex * ey * (g.nz - 2);
+  const int nint = (g.nx - 2) * (g.ny - 2) * (g.nz - 2);
   const float b = *L.lam;
-  for (int i = 0; i < K; i++) {
+  const float *cc = L.cc, *f = L.w0;
+  float* d = L.d;
+  for (int i = first; i < K; i++) {
     float alpha, beta;
     cheb_coef(b, i, alpha, beta);
     const float* xin = (i & 1) ? L.x2 : L.x;
     float* xout = (i & 1) ? L.x : L.x2;
-    for (int q = gtid; q < nint; q += nthr)
-      cheb_point(o, g, L.cc, L.w0, xin, xout, L.d, g.idx(1 + q % ex, 1 + (q / ex) % ey, 1 + q / (ex * ey)),
-                 alpha, beta);
+    for_points<2>(
+        nint, tid, [&](int q) { return interior_at(g, dx, dy, q); },
+        [&](int id) {
+          const float dg = o.c[OC][id] + cc[id];
+          const float xv = xin[id];
+          const float r = (f[id] + nb27(o, g, xin, id) - dg * xv) / dg;
+          const float dn = alpha * d[id] + beta * r;
+          return make_float2(dn, xv + dn);
+        },
+        [&](int id, float2 v) {
+          d[id] = v.x;
+          xout[id] = v.y;
+        });
     tail_sync<CLUSTER>();
   }
 }
 
-// restriction src (grid gs) -> level L's w0 (all points, boundary 0)
-__device__ void tail_restrict(Grid gs, const float* src, const TLev& L, bool zero_x, int gtid,
-                              int nthr) {
+// Restriction src (grid gs) -> level L's w0 (all points, boundary 0).  cheb0: also
+// the first Chebyshev step from x = 0, which needs no neighbour -- r = f / a_ii,
+// d = x2 = r / theta (the step the loop of tail_cheb would take over zeros);
+// otherwise x = 0.
+__device__ void tail_restrict(Grid gs, const float* src, const TLev& L, bool cheb0,
+                              TailTid tid) {
   const Grid gc = L.g;
   const int n = (int)gc.n();
-  for (int q = gtid; q < n; q += nthr) {
+  const float *oc = L.op[OC], *cc = L.cc;
+  float *w0 = L.w0, *x = L.x, *x2 = L.x2, *d = L.d;
+  float alpha, beta = 0.f;
+  if (cheb0) cheb_coef(*L.lam, 0, alpha, beta);
+  for (int q = tid.first(n); q < n; q += tid.n) {
     const int i = q % gc.nx, j = (q / gc.nx) % gc.ny, k = q / (gc.nx * gc.ny);
-    if (zero_x) L.x[q] = 0.f;
+    if (!cheb0) x[q] = 0.f;
     if (i == 0 || j == 0 || k == 0 || i == gc.nx - 1 || j == gc.ny - 1 || k == gc.nz - 1) {
-      L.w0[q] = 0.f;
+      w0[q] = 0.f;
       continue;
     }
     const int ii = 2 * i, jj = 2 * j, kk = 2 * k;
@@ -849,57 +930,118 @@ __device__ void tail_restrict(Grid gs, const float* src, const TLev& L, bool zer
           const float w = 1.f / (float)(1 << (abs(dx) + abs(dy) + abs(dz)));
           acc += w * src[gs.idx(ii + dx, jj + dy, kk + dz)];
         }
-    L.w0[q] = acc;
+    w0[q] = acc;
+    if (cheb0) {
+      const float dn = beta * (acc / (oc[q] + cc[q]));
+      d[q] = dn;
+      x2[q] = dn;
+    }
   }
 }
 
 // damping sums <x, w0> and <x, (A + cc) x> on level L
 template <int CLUSTER>
-__device__ void tail_damp(const TLev& L, int gtid, int nthr, double* sh, double* slots,
+__device__ void tail_damp(const TLev& L, TailTid tid, double* sh, double* slots,
                           int& phase, double& num, double& den) {
   const Grid g = L.g;
-  const int ex = g.nx - 2, ey = g.ny - 2;
-  const int nint = ex * ey * (g.nz - 2);
+  const unsigned dx = L.dx, dy = L.dy;
+  OpF o;
+#pragma unroll
+  for (int c = 0; c < 14; c++) o.c[c] = L.op[c];
+  o.nop = 14;
+  const int nint = (g.nx - 2) * (g.ny - 2) * (g.nz - 2);
+  const float *cc = L.cc, *x = L.x, *w0 = L.w0;
   double a = 0.0, b = 0.0;
-  for (int q = gtid; q < nint; q += nthr) {
-    const size_t id = g.idx(1 + q % ex, 1 + (q / ex) % ey, 1 + q / (ex * ey));
-    const float xv = L.x[id];
-    const float ax = (L.op[OC][id] + L.cc[id]) * xv - nb27t(L, L.x, id);
-    a += (double)xv * (double)L.w0[id];
-    b += (double)xv * (double)ax;
-  }
+  for_points<2>(
+      nint, tid, [&](int q) { return interior_at(g, dx, dy, q); },
+      [&](int id) {
+        const float xv = x[id];
+        return make_float2(w0[id], (o.c[OC][id] + cc[id]) * xv - nb27(o, g, x, id));
+      },
+      [&](int id, float2 v) {
+        const float xv = x[id];
+        a += (double)xv * (double)v.x;
+        b += (double)xv * (double)v.y;
+      });
   tail_sum2<CLUSTER>(a, b, sh, slots, phase);
   num = a;
   den = b;
+}
+
+// xf += xdamp * (trilinear interpolation of xc) on the interior of gf
+__device__ void tail_interp(Grid gc, const float* xc, Grid gf, unsigned dx, unsigned dy, float* xf,
+                            float xdamp, TailTid tid) {
+  const int ex = gf.nx - 2, ey = gf.ny - 2, nint = ex * ey * (gf.nz - 2);
+  for_points<2>(
+      nint, tid,
+      [&](int q) {
+        const int t = quotient(q, dx), k = quotient(t, dy);
+        // packed (i, j, k): 10 bits each hold the points of a cluster's levels
+        return (q - t * ex + 1) | (t - k * ey + 1) << 10 | (k + 1) << 20;
+      },
+      [&](int ijk) {
+        const int i = ijk & 1023, j = (ijk >> 10) & 1023, k = ijk >> 20;
+        const int ii = i >> 1, jj = j >> 1, kk = k >> 1;
+        const int oi = i & 1, oj = j & 1, ok = k & 1;
+        float w = 0.f;
+        for (int c = 0; c <= ok; c++)
+          for (int b = 0; b <= oj; b++)
+            for (int a = 0; a <= oi; a++) w += xc[gc.idx(ii + a, jj + b, kk + c)];
+        w *= 1.f / (float)(1 << (oi + oj + ok));
+        return make_float2(w, xf[gf.idx(i, j, k)]);
+      },
+      [&](int ijk, float2 v) {
+        xf[gf.idx(ijk & 1023, (ijk >> 10) & 1023, ijk >> 20)] = v.y + xdamp * v.x;
+      });
+}
+
+// The level table in shared memory (kTailLevels at most): the pointers of a pass
+// are then one shared load away, not one through an L1 that the barrier cleared.
+constexpr int kTailLevels = 16;
+__device__ __forceinline__ void tail_levels(TailArgs& A, TLev* sh) {
+  static_assert(sizeof(TLev) % 4 == 0 && sizeof(TailArgs) % 4 == 0, "copied by words");
+  const int words = (int)sizeof(TLev) / 4 * (A.last + 1);
+  for (int t = threadIdx.x; t < words; t += blockDim.x)
+    reinterpret_cast<unsigned*>(sh)[t] = reinterpret_cast<const unsigned*>(A.lev)[t];
+  A.lev = sh;
+  __syncthreads();
 }
 
 // One V-cycle from level A.first down to the dense level and back.  With
 // rhs_given the right-hand side of level first is already in its w0;
 // otherwise it is restricted from the residual of level first-1.
 template <int CLUSTER>
-__device__ void tail_cycle(const TailArgs& A, bool rhs_given, int gtid, int nthr, double* sh,
+__device__ void tail_cycle(const TailArgs& A, bool rhs_given, TailTid tid, double* sh,
                            double* slots, int& phase) {
   // down
   for (int l = A.first; l <= A.last; l++) {
     const TLev& L = A.lev[l];
+    const bool cheb0 = A.cheb > 0 && l != A.last && !(l == A.first && rhs_given);
     if (l == A.first && rhs_given) {
       const int n = (int)L.g.n();
-      for (int q = gtid; q < n; q += nthr) L.x[q] = 0.f;
+      for (int q = tid.first(n); q < n; q += tid.n) L.x[q] = 0.f;
     } else if (l == A.first) {
-      tail_restrict(A.gprev, A.rprev, L, true, gtid, nthr);
+      tail_restrict(A.gprev, A.rprev, L, cheb0, tid);
     } else {
-      tail_restrict(A.lev[l - 1].g, A.r, L, true, gtid, nthr);
+      tail_restrict(A.lev[l - 1].g, A.r, L, cheb0, tid);
     }
     tail_sync<CLUSTER>();
     if (l != A.last) {
-      if (A.cheb > 0) tail_cheb<CLUSTER>(L, gtid, nthr, A.cheb);
-      else tail_smooth<CLUSTER>(L, 0, gtid, nthr, A.nsweep);
+      if (A.cheb > 0) tail_cheb<CLUSTER>(L, tid, A.cheb, cheb0 ? 1 : 0);
+      else tail_smooth<CLUSTER>(L, 0, tid, A.nsweep);
       const Grid g = L.g;
-      const int ex = g.nx - 2, ey = g.ny - 2, nint = ex * ey * (g.nz - 2);
-      for (int q = gtid; q < nint; q += nthr) {
-        const size_t id = g.idx(1 + q % ex, 1 + (q / ex) % ey, 1 + q / (ex * ey));
-        A.r[id] = L.w0[id] + nb27t(L, L.x, id) - (L.op[OC][id] + L.cc[id]) * L.x[id];
-      }
+      const unsigned dx = L.dx, dy = L.dy;
+      const int nint = (g.nx - 2) * (g.ny - 2) * (g.nz - 2);
+      OpF o;
+#pragma unroll
+      for (int c = 0; c < 14; c++) o.c[c] = L.op[c];
+      o.nop = 14;
+      const float *cc = L.cc, *x = L.x, *w0 = L.w0;
+      float* r = A.r;
+      for_points<2>(
+          nint, tid, [&](int q) { return interior_at(g, dx, dy, q); },
+          [&](int id) { return w0[id] + nb27(o, g, x, id) - (o.c[OC][id] + cc[id]) * x[id]; },
+          [&](int id, float v) { r[id] = v; });
       tail_sync<CLUSTER>();
     }
   }
@@ -909,7 +1051,7 @@ __device__ void tail_cycle(const TailArgs& A, bool rhs_given, int gtid, int nthr
     const Grid g = L.g;
     const int ex = g.nx - 2, ey = g.ny - 2;
     const int lane = threadIdx.x & 31;
-    const int gw = gtid >> 5, nw = nthr >> 5;
+    const int gw = tid.round >> 5, nw = tid.n >> 5;
     for (int row = gw; row < A.nd; row += nw) {
       double t = 0.0;
       for (int c = lane; c < A.nd; c += 32)
@@ -925,41 +1067,35 @@ __device__ void tail_cycle(const TailArgs& A, bool rhs_given, int gtid, int nthr
     const TLev& C = A.lev[l + 1];
     const TLev& P = A.lev[l];
     double num, den;
-    tail_damp<CLUSTER>(C, gtid, nthr, sh, slots, phase, num, den);
+    tail_damp<CLUSTER>(C, tid, sh, slots, phase, num, den);
     const float xdamp = (float)(num / den);
-    const Grid gf = P.g;
-    const int ex = gf.nx - 2, ey = gf.ny - 2, nint = ex * ey * (gf.nz - 2);
-    for (int q = gtid; q < nint; q += nthr) {
-      const int i = 1 + q % ex, j = 1 + (q / ex) % ey, k = 1 + q / (ex * ey);
-      const int ii = i >> 1, jj = j >> 1, kk = k >> 1;
-      const int oi = i & 1, oj = j & 1, ok = k & 1;
-      float w = 0.f;
-      for (int c = 0; c <= ok; c++)
-        for (int b = 0; b <= oj; b++)
-          for (int a = 0; a <= oi; a++) w += C.x[C.g.idx(ii + a, jj + b, kk + c)];
-      w *= 1.f / (float)(1 << (oi + oj + ok));
-      P.x[gf.idx(i, j, k)] += xdamp * w;
-    }
+    tail_interp(C.g, C.x, P.g, P.dx, P.dy, P.x, xdamp, tid);
     tail_sync<CLUSTER>();
-    if (A.cheb > 0) tail_cheb<CLUSTER>(P, gtid, nthr, A.cheb);
-    else tail_smooth<CLUSTER>(P, 1, gtid, nthr, A.nsweep);
+    if (A.cheb > 0) tail_cheb<CLUSTER>(P, tid, A.cheb, 0);
+    else tail_smooth<CLUSTER>(P, 1, tid, A.nsweep);
   }
 }
 
+// The tail of one V-cycle.  Latency bounds it: a pass is a barrier (0.5 to 1.8 us
+// with the memory it orders) and a chain of L2 reads, on levels of a few thousand
+// points that give each thread one or none.  So a step's barriers were merged (the
+// first Chebyshev step goes with the restriction, the damping sums are pushed to
+// every CTA), the level table sits in shared memory, the loads of two points are in
+// flight together and small levels are spread over all the SMs: 33^3 grid (levels
+// 17^3 to 5^3) 58 -> 39 us, 49^3 77 -> 53, 225^3 91 -> 62, bitwise the same cycle.
 template <int CLUSTER>
 __global__ void __launch_bounds__(512) k_vcycle_tail(TailArgs A) {
   __shared__ double sh[64];
-  __shared__ double slots[4];
-  unsigned rank = 0;
-  if (CLUSTER > 1) rank = cg::this_cluster().block_rank();
-  const int gtid = rank * blockDim.x + threadIdx.x;
-  const int nthr = CLUSTER * blockDim.x;
+  __shared__ double slots[4 * CLUSTER];
+  __shared__ TLev levels[kTailLevels];
+  tail_levels(A, levels);
+  const TailTid tid = tail_tid<CLUSTER>();
   int phase = 0;
-  tail_cycle<CLUSTER>(A, false, gtid, nthr, sh, slots, phase);
+  tail_cycle<CLUSTER>(A, false, tid, sh, slots, phase);
   // damping sums for the first -> first-1 correction (done by the caller)
   double num, den;
-  tail_damp<CLUSTER>(A.lev[A.first], gtid, nthr, sh, slots, phase, num, den);
-  if (gtid == 0) {
+  tail_damp<CLUSTER>(A.lev[A.first], tid, sh, slots, phase, num, den);
+  if (tid.block == 0) {
     A.xnum[0] = num;
     A.xden[0] = den;
   }
@@ -1041,23 +1177,22 @@ struct ExactArgs {
 template <int CLUSTER>
 __global__ void __launch_bounds__(512) k_coarse_exact(ExactArgs E) {
   __shared__ double sh[64];
-  __shared__ double slots[4];
-  unsigned rank = 0;
-  if (CLUSTER > 1) rank = cg::this_cluster().block_rank();
-  const int gtid = rank * blockDim.x + threadIdx.x;
-  const int nthr = CLUSTER * blockDim.x;
+  __shared__ double slots[4 * CLUSTER];
+  __shared__ TLev levels[kTailLevels];
+  tail_levels(E.T, levels);
+  const TailTid tid = tail_tid<CLUSTER>();
   int phase = 0;
   const Grid g = E.g;
   const int ex = g.nx - 2, ey = g.ny - 2, nint = ex * ey * (g.nz - 2);
   const int n = (int)g.n();
   const TLev& L = E.T.lev[E.T.first];
-  for (int q = gtid; q < n; q += nthr) E.x[q] = 0.0;
+  for (int q = tid.first(n); q < n; q += tid.n) E.x[q] = 0.0;
   tail_sync<CLUSTER>();
   double bn = 0.0;
   int it = 0;
   for (;; it++) {
     double rr = 0.0, unused = 0.0;
-    for (int q = gtid; q < nint; q += nthr) {
+    for (int q = tid.first(nint); q < nint; q += tid.n) {
       const size_t id = g.idx(1 + q % ex, 1 + (q / ex) % ey, 1 + q / (ex * ey));
       const double v = E.b[id] + nb27g<double>(E.op, g, E.x, id) -
                        (E.op[OC][id] + E.cc[id]) * E.x[id];
@@ -1068,21 +1203,21 @@ __global__ void __launch_bounds__(512) k_coarse_exact(ExactArgs E) {
     const double rn = sqrt(rr);
     if (it == 0) bn = rn;
     if (bn == 0.0 || rn <= E.rtol * bn || it >= E.maxit) break;
-    for (int q = gtid; q < n; q += nthr) {
+    for (int q = tid.first(n); q < n; q += tid.n) {
       const int i = q % g.nx, j = (q / g.nx) % g.ny, k = q / (g.nx * g.ny);
       const bool bd = (i == 0 || j == 0 || k == 0 || i == g.nx - 1 || j == g.ny - 1 ||
                        k == g.nz - 1);
       L.w0[q] = bd ? 0.f : (float)E.r[q];
     }
     tail_sync<CLUSTER>();
-    tail_cycle<CLUSTER>(E.T, true, gtid, nthr, sh, slots, phase);
-    for (int q = gtid; q < nint; q += nthr) {
+    tail_cycle<CLUSTER>(E.T, true, tid, sh, slots, phase);
+    for (int q = tid.first(nint); q < nint; q += tid.n) {
       const size_t id = g.idx(1 + q % ex, 1 + (q / ex) % ey, 1 + q / (ex * ey));
       E.x[id] += (double)L.x[id];
     }
     tail_sync<CLUSTER>();
   }
-  if (gtid == 0) E.iters[0] = it;
+  if (tid.block == 0) E.iters[0] = it;
   // no CTA may exit while another can still read its shared memory
   tail_sync<CLUSTER>();
 }
@@ -1103,6 +1238,7 @@ __global__ void __launch_bounds__(512) k_coarse_exact(ExactArgs E) {
 struct BatchItem {
   TailArgs T;             // FP32 levels 1 .. coarsest (T.first = 1)
   Grid g;                 // fine grid
+  unsigned dx, dy, dh;    // div_const of nx - 2, ny - 2 and the points of a colour in a row
   const double* op[4];    // FP64 fine operator: oC oE oN uC
   const double* cc;
   const double* fc;
@@ -1119,123 +1255,142 @@ struct BatchItem {
   double* out;            // [0] corrections, [1] final relative residual, [2..] log
 };
 
-// one colour of the FP32 fine-level red-black GS (the update of k_gs7_f32)
+// one colour of the FP32 fine-level red-black GS (the update of k_gs7_f32); from
+// x = 0 (zero: the first colour of the first sweep) the neighbours are not read,
+// and the other colour is set to 0
 template <int CLUSTER>
-__device__ void batch_gs7(const BatchItem& B, int parity, int gtid, int nthr) {
+__device__ void batch_gs7(const BatchItem& B, unsigned dh, unsigned dy, int parity, bool zero,
+                          TailTid tid) {
   const Grid g = B.g;
   const int nx = g.nx, ny = g.ny, nz = g.nz;
-  const size_t sy = nx, sz = (size_t)nx * ny;
-  const int hr = (nx - 1) / 2;
-  const int nslots = hr * (ny - 2) * (nz - 2);
-  for (int q = gtid; q < nslots; q += nthr) {
-    const int m = q % hr;
-    const int j = 1 + (q / hr) % (ny - 2);
-    const int k = 1 + q / (hr * (ny - 2));
-    const int i = 1 + (((1 + j + k) & 1) != parity) + 2 * m;
-    if (i > nx - 2) continue;
-    const size_t id = g.idx(i, j, k);
-    const float* const* o = B.op32;
-    const float* x = B.e;
-    const float nb = o[ON][id] * x[id + sy] + o[ON][id - sy] * x[id - sy] + o[OE][id] * x[id + 1] +
-                     o[OE][id - 1] * x[id - 1] + o[UC][id - sz] * x[id - sz] +
-                     o[UC][id] * x[id + sz];
-    B.e[id] = (B.w0[id] + nb) / (o[OC][id] + B.cc32[id]);
-  }
+  const int sy = nx, sz = nx * ny;
+  const int hr = (nx - 1) / 2, ey = ny - 2;
+  const int nslots = hr * ey * (nz - 2);
+  const float *oC = B.op32[OC], *oN = B.op32[ON], *oE = B.op32[OE], *uC = B.op32[UC];
+  const float *cc = B.cc32, *w0 = B.w0;
+  float* x = B.e;
+  for_points<4>(
+      nslots, tid,
+      [&](int q) {
+        const int t = quotient(q, dh), k = quotient(t, dy) + 1;
+        const int m = q - t * hr, j = t - (k - 1) * ey + 1;
+        const int off = ((1 + j + k) & 1) != parity;
+        const int i = 1 + off + 2 * m;
+        if (zero) x[(k * ny + j) * nx + 2 - off + 2 * m] = 0.f;  // a boundary's 0 stays 0
+        return i > nx - 2 ? -1 : (k * ny + j) * nx + i;
+      },
+      [&](int id) {
+        float nb = 0.f;
+        if (!zero)
+          nb = oN[id] * x[id + sy] + oN[id - sy] * x[id - sy] + oE[id] * x[id + 1] +
+               oE[id - 1] * x[id - 1] + uC[id - sz] * x[id - sz] + uC[id] * x[id + sz];
+        return (w0[id] + nb) / (oC[id] + cc[id]);
+      },
+      [&](int id, float v) { x[id] = v; });
   tail_sync<CLUSTER>();
 }
 
+// Bounded by the L2's rate to the SMs of one cluster at 65^3 and by latency at 33^3.
+// First colour from zero without reading the neighbours, points by multiplication
+// instead of division, four points' loads in flight, and the tail above: a batch of
+// five each of 33^3, 49^3 and 65^3 11.8 -> 10.6 ms, the same bits.
 template <int CLUSTER>
 __global__ void __launch_bounds__(512) k_batch_solve(const BatchItem* __restrict__ items) {
   __shared__ double sh[64];
-  __shared__ double slots[4];
-  const BatchItem& B = items[blockIdx.x / CLUSTER];
-  const unsigned rank = cg::this_cluster().block_rank();
-  const int gtid = rank * blockDim.x + threadIdx.x;
-  const int nthr = CLUSTER * blockDim.x;
+  __shared__ double slots[4 * CLUSTER];
+  __shared__ TLev levels[kTailLevels];
+  __shared__ __align__(16) unsigned item[sizeof(BatchItem) / 4];
+  for (int t = threadIdx.x; t < (int)sizeof(BatchItem) / 4; t += blockDim.x)
+    item[t] = reinterpret_cast<const unsigned*>(items + blockIdx.x / CLUSTER)[t];
+  __syncthreads();
+  const BatchItem& B = *reinterpret_cast<const BatchItem*>(item);
+  TailArgs T = B.T;
+  tail_levels(T, levels);
+  const TailTid tid = tail_tid<CLUSTER>();
   int phase = 0;
   const Grid g = B.g;
   const int nx = g.nx, ny = g.ny;
   const int ex = nx - 2, ey = ny - 2, nint = ex * ey * (g.nz - 2);
   const int n = (int)g.n();
-  const size_t sy = nx, sz = (size_t)nx * ny;
-  auto interior = [&](int q) { return g.idx(1 + q % ex, 1 + (q / ex) % ey, 1 + q / (ex * ey)); };
+  const int sy = nx, sz = nx * ny;
+  const unsigned dx = B.dx, dy = B.dy;
+  auto interior = [&](int q) { return interior_at(g, dx, dy, q); };
 
   // x = 0; ||f||_1 (Vxnrm1 on the interior)
   double fs = 0.0, u2 = 0.0;
-  for (int q = gtid; q < n; q += nthr) B.x[q] = 0.0;
-  for (int q = gtid; q < nint; q += nthr) fs += fabs(B.fc[interior(q)]);
+  for (int q = tid.first(n); q < n; q += tid.n) B.x[q] = 0.0;
+  for (int q = tid.first(nint); q < nint; q += tid.n) fs += fabs(B.fc[interior(q)]);
   tail_sum2<CLUSTER>(fs, u2, sh, slots, phase);
   const double rsden = (fs == 0.0) ? 1.0 : fs;
   // FP64 residual r = f - (A + cc) x -> FP32 right-hand side, and ||r||_1
   auto residual = [&]() {
     double acc = 0.0, unused = 0.0;
-    for (int q = gtid; q < nint; q += nthr) {
-      const size_t id = interior(q);
-      const double* const* o = B.op;
-      const double* x = B.x;
-      const double r = B.fc[id] + o[ON][id] * x[id + sy] + o[ON][id - sy] * x[id - sy] +
-                       o[OE][id] * x[id + 1] + o[OE][id - 1] * x[id - 1] +
-                       o[UC][id - sz] * x[id - sz] + o[UC][id] * x[id + sz] -
-                       (o[OC][id] + B.cc[id]) * x[id];
-      B.w0[id] = (float)r;
-      acc += fabs(r);
-    }
+    const double *oC = B.op[OC], *oN = B.op[ON], *oE = B.op[OE], *uC = B.op[UC];
+    const double *x = B.x, *f = B.fc, *cc = B.cc;
+    float* w0 = B.w0;
+    for_points<2>(
+        nint, tid, interior,
+        [&](int id) {
+          return f[id] + oN[id] * x[id + sy] + oN[id - sy] * x[id - sy] + oE[id] * x[id + 1] +
+                 oE[id - 1] * x[id - 1] + uC[id - sz] * x[id - sz] + uC[id] * x[id + sz] -
+                 (oC[id] + cc[id]) * x[id];
+        },
+        [&](int id, double r) {
+          w0[id] = (float)r;
+          acc += fabs(r);
+        });
     tail_sum2<CLUSTER>(acc, unused, sh, slots, phase);
     return acc;
   };
   double rs = residual();
-  if (gtid == 0 && B.nlog > 0) B.out[2] = rs / rsden;
+  if (tid.block == 0 && B.nlog > 0) B.out[2] = rs / rsden;
   int it = 0;
   while (it < B.itmax && rs / rsden > B.errtol) {
     // FP32 V-cycle on A e = w0
-    for (int q = gtid; q < n; q += nthr) B.e[q] = 0.f;
-    tail_sync<CLUSTER>();
     for (int sw = 0; sw < B.fine_sweeps; sw++) {
-      batch_gs7<CLUSTER>(B, 1, gtid, nthr);
-      batch_gs7<CLUSTER>(B, 0, gtid, nthr);
+      batch_gs7<CLUSTER>(B, B.dh, dy, 1, sw == 0, tid);
+      batch_gs7<CLUSTER>(B, B.dh, dy, 0, false, tid);
     }
-    for (int q = gtid; q < nint; q += nthr) {
-      const size_t id = interior(q);
-      const float* const* o = B.op32;
-      const float* x = B.e;
-      const float nb = o[ON][id] * x[id + sy] + o[ON][id - sy] * x[id - sy] +
-                       o[OE][id] * x[id + 1] + o[OE][id - 1] * x[id - 1] +
-                       o[UC][id - sz] * x[id - sz] + o[UC][id] * x[id + sz];
-      B.r[id] = B.w0[id] + nb - (o[OC][id] + B.cc32[id]) * x[id];
+    {
+      const float *oC = B.op32[OC], *oN = B.op32[ON], *oE = B.op32[OE], *uC = B.op32[UC];
+      const float *x = B.e, *w0 = B.w0, *cc = B.cc32;
+      float* r = B.r;
+      for_points<4>(
+          nint, tid, interior,
+          [&](int id) {
+            const float nb = oN[id] * x[id + sy] + oN[id - sy] * x[id - sy] + oE[id] * x[id + 1] +
+                             oE[id - 1] * x[id - 1] + uC[id - sz] * x[id - sz] +
+                             uC[id] * x[id + sz];
+            return w0[id] + nb - (oC[id] + cc[id]) * x[id];
+          },
+          [&](int id, float v) { r[id] = v; });
     }
     tail_sync<CLUSTER>();
-    tail_cycle<CLUSTER>(B.T, false, gtid, nthr, sh, slots, phase);
-    const TLev& C = B.T.lev[1];
+    tail_cycle<CLUSTER>(T, false, tid, sh, slots, phase);
+    const TLev& C = T.lev[1];
     double num, den;
-    tail_damp<CLUSTER>(C, gtid, nthr, sh, slots, phase, num, den);
+    tail_damp<CLUSTER>(C, tid, sh, slots, phase, num, den);
     const float xdamp = (float)(num / den);
-    for (int q = gtid; q < nint; q += nthr) {
-      const int i = 1 + q % ex, j = 1 + (q / ex) % ey, k = 1 + q / (ex * ey);
-      const int ii = i >> 1, jj = j >> 1, kk = k >> 1;
-      const int oi = i & 1, oj = j & 1, ok = k & 1;
-      float w = 0.f;
-      for (int c = 0; c <= ok; c++)
-        for (int b = 0; b <= oj; b++)
-          for (int a = 0; a <= oi; a++) w += C.x[C.g.idx(ii + a, jj + b, kk + c)];
-      w *= 1.f / (float)(1 << (oi + oj + ok));
-      B.e[g.idx(i, j, k)] += xdamp * w;
-    }
+    tail_interp(C.g, C.x, g, dx, dy, B.e, xdamp, tid);
     tail_sync<CLUSTER>();
     for (int sw = 0; sw < B.fine_sweeps; sw++) {
-      batch_gs7<CLUSTER>(B, 0, gtid, nthr);
-      batch_gs7<CLUSTER>(B, 1, gtid, nthr);
+      batch_gs7<CLUSTER>(B, B.dh, dy, 0, false, tid);
+      batch_gs7<CLUSTER>(B, B.dh, dy, 1, false, tid);
     }
-    for (int q = gtid; q < nint; q += nthr) {
-      const size_t id = interior(q);
-      B.x[id] += (double)B.e[id];
+    {
+      double* x = B.x;
+      const float* e = B.e;
+      for_points<4>(
+          nint, tid, interior, [&](int id) { return x[id] + (double)e[id]; },
+          [&](int id, double v) { x[id] = v; });
     }
     tail_sync<CLUSTER>();
     rs = residual();
     it++;
-    if (gtid == 0 && it < B.nlog) B.out[2 + it] = rs / rsden;
+    if (tid.block == 0 && it < B.nlog) B.out[2 + it] = rs / rsden;
     if (!(rs == rs)) break;  // non-finite: reported by the host
   }
-  if (gtid == 0) {
+  if (tid.block == 0) {
     B.out[0] = (double)it;
     B.out[1] = rs / rsden;
   }
@@ -1526,8 +1681,12 @@ int mixed_setup_from(pmgb_solver* s, int lo) {
   }
   if (!dalloc64(&m->dense, (size_t)m->nd * m->nd) || !dalloc64(&m->dvec, m->nd)) return 0;
   CKM(cudaMalloc(&m->dinfo, sizeof(int) * 4));
-  // levels small enough for one cluster run in the tail kernel
-  // the exact coarse solve of the FP64 path always runs its levels in one
+  // Levels small enough for one cluster run in the tail kernel: 16 SMs take a pass
+  // over 33^3 points at about 8 us (their share of the L2's bandwidth bounds it),
+  // a launch on all SMs at 3 us, while 25^3 and below take 2 to 3 us in the cluster
+  // with the barrier.  Limit 70000 -> 20000: LPBE solves of 65^3 1.43 -> 1.30 ms,
+  // 129^3 3.06 -> 2.90, NPBE 161^3 8.11 -> 7.52.
+  // The exact coarse solve of the FP64 path always runs its levels in one
   // cluster; the mixed V-cycle does from the first level under the limit
   m->tail_first = (lo > 0) ? lo : 0;
   for (int l = 1; lo == 0 && l < nl; l++) {
@@ -1537,10 +1696,12 @@ int mixed_setup_from(pmgb_solver* s, int lo) {
       break;
     }
   }
-  if (m->tail_first > 0) {
+  {
     std::vector<TLev> tl(nl);
     for (int l = 0; l < nl; l++) {
       tl[l].g = m->lev[l].g;
+      tl[l].dx = div_const(m->lev[l].g.nx - 2);
+      tl[l].dy = div_const(m->lev[l].g.ny - 2);
       for (int c = 0; c < 14; c++) tl[l].op[c] = m->lev[l].op[c];
       tl[l].cc = m->lev[l].cc;
       tl[l].w0 = m->lev[l].w0;
@@ -2173,19 +2334,14 @@ extern "C" int pmgb_batch_solve(pmgb_solver* const* solvers, int n, void* cuda_s
   for (int b = 0; b < n; b++) {
     pmgb_solver* s = solvers[b];
     if (!s->built && !solver_build(s)) return 0;
-    // the persistent kernel runs every level from 1 down in its cluster: a
-    // calculation tuned to keep level 1 outside the one-cluster tail takes
-    // a tail limit that holds it (the FP32 hierarchy is rebuilt once)
-    if (s->nlev > 1) {
-      const Grid g1 = s->lev[1].g;
-      const int need = (g1.nx - 2) * (g1.ny - 2) * (g1.nz - 2);
-      if (need <= kBatchTailMax && s->tune[PMGB_TUNE_TAIL_MAX_POINTS] < need &&
-          !pmgb_solver_set_tuning(s, PMGB_TUNE_TAIL_MAX_POINTS, need))
-        return 0;
-    }
     if (!mixed_setup(s) || !mixed_refresh(s)) return 0;
     if (!s->mixed->cc_ready && !mixed_set_cc(s, 0)) return 0;
-    if (s->mixed->tail_first != 1) {
+    // the persistent kernel runs every level from 1 down in its cluster, whatever
+    // level the calculation's own V-cycle begins its tail at
+    const Grid g1 = s->nlev > 1 ? s->lev[1].g : s->g;
+    const size_t n1 = (size_t)(g1.nx - 2) * (g1.ny - 2) * (g1.nz - 2);
+    if (s->nlev < 2 ||
+        n1 > (size_t)std::max(kBatchTailMax, s->tune[PMGB_TUNE_TAIL_MAX_POINTS])) {
       set_error("pmgb_batch_solve: calculation %d (%dx%dx%d) is too large for one cluster "
                 "(its level 1 exceeds the tail limit)", b, s->p.nx, s->p.ny, s->p.nz);
       return 0;
@@ -2243,6 +2399,9 @@ extern "C" int pmgb_batch_solve(pmgb_solver* const* solvers, int n, void* cuda_s
     B.T.xnum = s->scal + S_TMP;
     B.T.xden = s->scal + S_TMP;
     B.g = s->g;
+    B.dx = div_const(s->g.nx - 2);
+    B.dy = div_const(s->g.ny - 2);
+    B.dh = div_const((s->g.nx - 1) / 2);
     for (int c = 0; c < 4; c++) {
       B.op[c] = s->lev[0].op[c];
       B.op32[c] = m->lev[0].op[c];

@@ -240,7 +240,9 @@ int pmgb_solve_molecule(const pmgb_params *params, int precision, int natoms,
 #define PMGB_TUNE_GS27_CLUSTER_MID 7   /* the same as key 2 for levels with 28-59 interior
                                           points per axis (0 = 8) */
 #define PMGB_TUNE_TAIL_MAX_POINTS 8    /* mixed: largest level (interior points) run inside
-                                          the one-cluster V-cycle tail (default 70000) */
+                                          the one-cluster V-cycle tail (default 20000);
+                                          pmgb_batch_solve runs its levels in one
+                                          cluster whatever this says */
 #define PMGB_TUNE_MC_COOPERATIVE 9    /* mixed: 8-colour GS on levels above 200000 interior
                                           points as one cooperative launch per smoothing call
                                           (1) instead of one launch per colour (0) */
