@@ -280,7 +280,7 @@ __device__ __forceinline__ float nb7(const OpF& o, Grid g, const float* x, size_
          o.c[OE][id - 1] * x[id - 1] + o.c[UC][id - sz] * x[id - sz] + o.c[UC][id] * x[id + sz];
 }
 
-__global__ void k_gs7_f32(Grid g, OpF o, const float* __restrict__ cc,
+__global__ void k_gs7_f32(Grid g, OpF o, const float* __restrict__ D,
                           const float* __restrict__ fc, float* x, int parity) {
   const int nx = g.nx, ny = g.ny, nz = g.nz;
   const int hr = (nx - 1) / 2;
@@ -294,22 +294,47 @@ __global__ void k_gs7_f32(Grid g, OpF o, const float* __restrict__ cc,
     const int i = 1 + (((1 + j + k) & 1) != parity) + 2 * m;
     if (i > nx - 2) continue;
     const size_t id = g.idx(i, j, k);
-    x[id] = (fc[id] + nb7(o, g, x, id)) / (o.c[OC][id] + cc[id]);
+    x[id] = (fc[id] + nb7(o, g, x, id)) / D[id];
   }
 }
 
-// r = f - (A + cc) x on interior points (7- or 27-point)
-__global__ void k_resid_f32(Grid g, OpF o, const float* __restrict__ cc,
-                            const float* __restrict__ fc, const float* __restrict__ x, float* r) {
-  const int nx = g.nx, ny = g.ny, nz = g.nz;
-  const size_t nint = (size_t)(nx - 2) * (ny - 2) * (nz - 2);
+// The first colour pass from x = 0: f / D at the points of the colour, 0 at the
+// others, so neither x nor the couplings are read and x needs no clearing before.
+__global__ void k_gs7_f32_first(Grid g, const float* __restrict__ D, const float* __restrict__ fc,
+                                float* __restrict__ x, int parity) {
+  const size_t nint = (size_t)(g.nx - 2) * (g.ny - 2) * (g.nz - 2);
   for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < nint;
        q += (size_t)gridDim.x * blockDim.x) {
     int i, j, k;
-    interior_ijk(q, nx, ny, i, j, k);
+    interior_ijk(q, g.nx, g.ny, i, j, k);
     const size_t id = g.idx(i, j, k);
-    const float nb = (o.nop == 4) ? nb7(o, g, x, id) : nb27(o, g, x, id);
-    r[id] = fc[id] + nb - (o.c[OC][id] + cc[id]) * x[id];
+    x[id] = ((i + j + k) & 1) == parity ? fc[id] / D[id] : 0.f;
+  }
+}
+
+// r = f - (A + cc) x on interior points of a 7-point level, D = oC + cc
+__global__ void k_resid7_f32(Grid g, OpF o, const float* __restrict__ D,
+                             const float* __restrict__ fc, const float* __restrict__ x, float* r) {
+  const size_t nint = (size_t)(g.nx - 2) * (g.ny - 2) * (g.nz - 2);
+  for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < nint;
+       q += (size_t)gridDim.x * blockDim.x) {
+    int i, j, k;
+    interior_ijk(q, g.nx, g.ny, i, j, k);
+    const size_t id = g.idx(i, j, k);
+    r[id] = fc[id] + nb7(o, g, x, id) - D[id] * x[id];
+  }
+}
+
+// r = f - (A + cc) x on interior points of a 27-point level
+__global__ void k_resid_f32(Grid g, OpF o, const float* __restrict__ cc,
+                            const float* __restrict__ fc, const float* __restrict__ x, float* r) {
+  const size_t nint = (size_t)(g.nx - 2) * (g.ny - 2) * (g.nz - 2);
+  for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < nint;
+       q += (size_t)gridDim.x * blockDim.x) {
+    int i, j, k;
+    interior_ijk(q, g.nx, g.ny, i, j, k);
+    const size_t id = g.idx(i, j, k);
+    r[id] = fc[id] + nb27(o, g, x, id) - (o.c[OC][id] + cc[id]) * x[id];
   }
 }
 
@@ -395,15 +420,24 @@ __global__ void __launch_bounds__(256) k_gs27_mc_coop(Grid g, OpF o, const float
     }
 }
 
-__global__ void k_restrict_f32(Grid gf, const float* __restrict__ xin, Grid gc, float* xout) {
+// The restriction of xin to level C's right-hand side w0 (0 on the boundary).  With
+// x2 given also the first Chebyshev step from x = 0, r = w0 / a_ii, d = x2 = r / theta
+// (k_cheb_step over zeros, without the pass over the couplings); without, x (if given)
+// is set to 0.
+__global__ void k_restrict_f32(Grid gf, const float* __restrict__ xin, Grid gc, float* w0,
+                               const float* __restrict__ oc, const float* __restrict__ cc,
+                               const float* __restrict__ lam, float* x, float* x2, float* d) {
   const int cx = gc.nx, cy = gc.ny, cz = gc.nz;
   const size_t n = gc.n();
+  float alpha, beta = 0.f;
+  if (x2) cheb_coef(*lam, 0, alpha, beta);
   for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < n;
        q += (size_t)gridDim.x * blockDim.x) {
     int i, j, k;
     split3(q, cx, cy, i, j, k);
+    if (!x2 && x) x[q] = 0.f;
     if (i == 0 || j == 0 || k == 0 || i == cx - 1 || j == cy - 1 || k == cz - 1) {
-      xout[q] = 0.f;
+      w0[q] = 0.f;
       continue;
     }
     const int ii = 2 * i, jj = 2 * j, kk = 2 * k;
@@ -417,7 +451,12 @@ __global__ void k_restrict_f32(Grid gf, const float* __restrict__ xin, Grid gc, 
           const float w = 1.f / (float)(1 << (abs(dx) + abs(dy) + abs(dz)));
           acc += w * xin[gf.idx(ii + dx, jj + dy, kk + dz)];
         }
-    xout[q] = acc;
+    w0[q] = acc;
+    if (x2) {
+      const float dn = beta * (acc / (oc[q] + cc[q]));
+      d[q] = dn;
+      x2[q] = dn;
+    }
   }
 }
 
@@ -1485,48 +1524,65 @@ Gs7Rb<float> rb_f32(const MLevel& F, const float* d32, const int* tune) {
   return a;
 }
 
-// The fine-level FP32 smoothing: tune[11] red-black sweeps, then (r given)
-// the residual.  tune[5] == 2 runs single-pass sweeps out of place
-// (x -> xs -> x ...; after an odd count xs is copied back); otherwise one
-// launch per colour.  k counts the kernels launched.
+// The fine-level FP32 smoothing: tune[11] red-black sweeps, from x = 0 (zero) or
+// from x, then (r given) the residual.  Memory bounds a colour pass, the L2's up to
+// 129^3 and HBM above, so the first pass from zero only writes, the diagonal is one
+// array (oC + cc, as the single-pass sweep has it), and above kSinglePassMin points
+// (tune[5] == 0), or for tune[5] == 2, the other sweeps take a single pass out of
+// place (x -> xs -> x ...; after an odd count xs is copied back): two colour passes
+// 21.6 us and a single pass 22.7 at 129^3, 41.5 and 36.9 at 161^3, 118 and 89 at
+// 225^3.  An LPBE solve of 225^3 11.8 -> 10.6 ms and of 65^3 1.30 -> 1.22, the same
+// bits.  k counts the kernels launched.
+constexpr size_t kSinglePassMin = 3000000;
+
 cudaError_t gs7_f32(cudaStream_t st, const MLevel& F, float* x, float* r, int first_parity,
-                    float* xs, const float* d32, const int* tune, long long& k) {
+                    float* xs, const float* d32, bool zero, const int* tune, long long& k) {
   const int nsweep = tune[11];
-  if (tune[5] == 2 && xs && d32 && (F.g.nx & 1) && (F.g.ny & 1)) {
+  const size_t fint = (size_t)(F.g.nx - 2) * (F.g.ny - 2) * (F.g.nz - 2);
+  const OpF fo = opf(F);
+  const size_t nslots = (size_t)((F.g.nx - 1) / 2) * (F.g.ny - 2) * (F.g.nz - 2);
+  cudaError_t e = cudaSuccess;
+  auto colour = [&](int c) {
+    k_gs7_f32<<<blocks_for(nslots), kThreads, 0, st>>>(F.g, fo, d32, F.w0, x, c);
+    k++;
+  };
+  int sw = 0;
+  if (zero && nsweep > 0) {
+    k_gs7_f32_first<<<blocks_for(fint), kThreads, 0, st>>>(F.g, d32, F.w0, x, first_parity);
+    k++;
+    colour(1 - first_parity);
+    sw = 1;
+  } else if (zero) {
+    e = cudaMemsetAsync(x, 0, F.g.n() * sizeof(float), st);
+  }
+  const bool single = tune[5] == 2 ? (F.g.nx & 1) && (F.g.ny & 1)
+                                   : tune[5] == 0 && fint >= kSinglePassMin &&
+                                         gs7_rb_suits<float>(F.g.nx, F.g.ny, F.g.n(), tune[12]);
+  if (single) {
     Gs7Rb<float> a = rb_f32(F, d32, tune);
-    float* buf[2] = {x, xs};
-    cudaError_t e = cudaSuccess;
-    for (int sw = 0; sw < nsweep && e == cudaSuccess; sw++) {
-      a.xin = buf[sw & 1];
-      a.xout = buf[(sw + 1) & 1];
+    float *xin = x, *xout = xs;
+    for (; sw < nsweep && e == cudaSuccess; sw++) {
+      a.xin = xin;
+      a.xout = xout;
       e = launch_gs7_rb<float>(st, a, first_parity, tune[12]);
       k++;
+      std::swap(xin, xout);
     }
-    if (e == cudaSuccess && (nsweep & 1))
+    if (e == cudaSuccess && xin != x)
       e = cudaMemcpyAsync(x, xs, F.g.n() * sizeof(float), cudaMemcpyDeviceToDevice, st);
-    if (r && e == cudaSuccess) {
-      const size_t fint = (size_t)(F.g.nx - 2) * (F.g.ny - 2) * (F.g.nz - 2);
-      k_resid_f32<<<blocks_for(fint), kThreads, 0, st>>>(F.g, opf(F), F.cc, F.w0, x, r);
-      k++;
-      e = cudaGetLastError();
+  } else {
+    for (; sw < nsweep; sw++) {
+      colour(first_parity);
+      colour(1 - first_parity);
     }
-    return e;
   }
-  // colour passes: the sweeps, then the residual
-  const size_t nslots = (size_t)((F.g.nx - 1) / 2) * (F.g.ny - 2) * (F.g.nz - 2);
-  const OpF fo = opf(F);
-  for (int sw = 0; sw < nsweep; sw++) {
-    k_gs7_f32<<<blocks_for(nslots), kThreads, 0, st>>>(F.g, fo, F.cc, F.w0, x, first_parity);
-    k_gs7_f32<<<blocks_for(nslots), kThreads, 0, st>>>(F.g, fo, F.cc, F.w0, x,
-                                                       1 - first_parity);
-    k += 2;
-  }
-  if (r) {
-    const size_t fint = (size_t)(F.g.nx - 2) * (F.g.ny - 2) * (F.g.nz - 2);
-    k_resid_f32<<<blocks_for(fint), kThreads, 0, st>>>(F.g, fo, F.cc, F.w0, x, r);
+  if (e == cudaSuccess) e = cudaGetLastError();
+  if (r && e == cudaSuccess) {
+    k_resid7_f32<<<blocks_for(fint), kThreads, 0, st>>>(F.g, fo, d32, F.w0, x, r);
     k++;
+    e = cudaGetLastError();
   }
-  return cudaGetLastError();
+  return e;
 }
 
 // FP32 D = oC + cc inside, 1 on the boundary
@@ -1882,8 +1938,8 @@ int mixed_set_cc(pmgb_solver* s, int newton, int defer_check = 0) {
   // the FP32 Helmholtz terms of all levels in one launch
   conv.flush();
   MLevel& F = m->lev[0];
-  if (m->d32 && s->tune[PMGB_TUNE_GS7_COLOUR_PASSES] == 2) {
-    // the FP32 single-pass sweep's divisor
+  if (m->d32) {
+    // the fine level's divisor, one array for the sweeps and the residual to read
     k_diag_f32<<<blocks_for(F.g.n()), kThreads, 0, st>>>(F.g, F.op[OC], F.cc, m->d32);
     note_launches(1);
   }
@@ -1913,13 +1969,13 @@ int cheb_degree(const int* tune) {
 
 // smoothing of a 27-point FP32 level outside the tail: K Chebyshev steps
 // (one launch each) or the 8-colour Gauss-Seidel
-int smooth27(cudaStream_t st, MLevel& L, MixedState* m, int l, int reverse, long long& k,
-             const int* tune) {
+int smooth27(cudaStream_t st, MLevel& L, MixedState* m, int l, int first, int reverse,
+             long long& k, const int* tune) {
   const int K = cheb_degree(tune);
   if (K == 0 || !L.x2) return gs27_mc(st, L, L.x, tune[10], reverse, k, tune[9]);
   const size_t nint = (size_t)(L.g.nx - 2) * (L.g.ny - 2) * (L.g.nz - 2);
   const OpF o = opf(L);
-  for (int i = 0; i < K; i++) {
+  for (int i = first; i < K; i++) {
     k_cheb_step<<<blocks_for(nint), kThreads, 0, st>>>(L.g, o, L.cc, L.w0, (i & 1) ? L.x2 : L.x,
                                                        (i & 1) ? L.x : L.x2, L.d, m->lam + l, i);
     k++;
@@ -1975,20 +2031,21 @@ int mixed_cycle_body(pmgb_solver* s, const double* cc64, const double* fc64, dou
   MLevel& F = m->lev[0];
   const OpF fo = opf(F);
   const size_t fint = (size_t)(F.g.nx - 2) * (F.g.ny - 2) * (F.g.nz - 2);
-  CKM(cudaMemsetAsync(F.x, 0, F.g.n() * sizeof(float), st));
-  if (gs7_f32(st, F, F.x, m->r, 1, m->xs, m->d32, s->tune, k) != cudaSuccess) {
+  if (gs7_f32(st, F, F.x, m->r, 1, m->xs, m->d32, true, s->tune, k) != cudaSuccess) {
     set_error("FP32 fine smoother launch failed");
     return 0;
   }
   const int tf = m->tail_first > 0 ? m->tail_first : nl;
   for (int l = 1; l < tf; l++) {
     MLevel& C = m->lev[l];
-    k_restrict_f32<<<blocks_for(C.g.n()), kThreads, 0, st>>>(m->lev[l - 1].g, m->r, C.g,
-                                                             C.w0);
+    const bool last = l == nl - 1;
+    const bool cheb0 = !last && cheb_degree(s->tune) > 0 && C.x2;
+    k_restrict_f32<<<blocks_for(C.g.n()), kThreads, 0, st>>>(
+        m->lev[l - 1].g, m->r, C.g, C.w0, C.op[OC], C.cc, m->lam + l, last ? nullptr : C.x,
+        cheb0 ? C.x2 : nullptr, C.d);
     k++;
-    if (l != nl - 1) {
-      CKM(cudaMemsetAsync(C.x, 0, C.g.n() * sizeof(float), st));
-      if (!smooth27(st, C, m, l, 0, k, s->tune)) return 0;
+    if (!last) {
+      if (!smooth27(st, C, m, l, cheb0 ? 1 : 0, 0, k, s->tune)) return 0;
       const size_t cint = (size_t)(C.g.nx - 2) * (C.g.ny - 2) * (C.g.nz - 2);
       k_resid_f32<<<blocks_for(cint), kThreads, 0, st>>>(C.g, opf(C), C.cc, C.w0, C.x, m->r);
       k++;
@@ -2019,12 +2076,12 @@ int mixed_cycle_body(pmgb_solver* s, const double* cc64, const double* fc64, dou
         C.g, C.x, P.g, P.x, s->scal + S_XNUM_L + (l & 15), s->scal + S_XDEN_L + (l & 15));
     k += 1;
     if (l == 0) {
-      if (gs7_f32(st, F, F.x, nullptr, 0, m->xs, m->d32, s->tune, k) != cudaSuccess) {
+      if (gs7_f32(st, F, F.x, nullptr, 0, m->xs, m->d32, false, s->tune, k) != cudaSuccess) {
         set_error("FP32 fine smoother launch failed");
         return 0;
       }
     } else {
-      if (!smooth27(st, P, m, l, 1, k, s->tune)) return 0;
+      if (!smooth27(st, P, m, l, 0, 1, k, s->tune)) return 0;
     }
   }
   // x64 += e ; r = f - (A + cc) x64 (FP64) -> FP32 rhs ; ||r||_1
@@ -2139,16 +2196,16 @@ int mixed_newton_inner(pmgb_solver* s, double errtol_s) {
   return refine(s, 1, F.cp, F.rhs, F.xt, errtol_s, 1000, 1, &it);
 }
 
-// One FP32 fine-level half-sweep for kernel timing; 6 FP32 arrays read and
-// x read/written: 14 B per point per half-sweep.
+// One FP32 fine-level half-sweep for kernel timing; 5 FP32 arrays read and
+// x read/written: 12 B per point per half-sweep.
 int mixed_time_gs7(pmgb_solver* s, int parity, double* bytes) {
   if (!mixed_setup(s) || !mixed_refresh(s)) return 0;
   MixedState* m = s->mixed;
   MLevel& F = m->lev[0];
   const size_t nslots = (size_t)((F.g.nx - 1) / 2) * (F.g.ny - 2) * (F.g.nz - 2);
-  k_gs7_f32<<<blocks_for(nslots), kThreads, 0, s->stream>>>(F.g, opf(F), F.cc, F.w0, F.x,
+  k_gs7_f32<<<blocks_for(nslots), kThreads, 0, s->stream>>>(F.g, opf(F), m->d32, F.w0, F.x,
                                                             parity);
-  *bytes = 14.0 * (double)(F.g.nx - 2) * (F.g.ny - 2) * (F.g.nz - 2);
+  *bytes = 12.0 * (double)(F.g.nx - 2) * (F.g.ny - 2) * (F.g.nz - 2);
   return 1;
 }
 

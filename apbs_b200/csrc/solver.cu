@@ -1610,7 +1610,8 @@ extern "C" int pmgb_time_kernel(pmgb_solver* s, int which, int reps, double* ms,
   Level& F = s->lev[0];
   const double fint = (double)(F.g.nx - 2) * (F.g.ny - 2) * (F.g.nz - 2);
   double b = 0.0;
-  if (which == PMGB_K_GS7_SWEEP_FP32 && !mixed_prepare_sweep(s)) return 0;
+  if ((which == PMGB_K_GS7_SWEEP_FP32 || which == PMGB_K_GS7_FP32) && !mixed_prepare_sweep(s))
+    return 0;
   if (which == PMGB_K_GS27_WAVE) gs27_pack(s, 0);
   CK(cudaStreamSynchronize(st));
   CK(cudaEventRecord(s->ev[6], st));
