@@ -526,7 +526,7 @@ __global__ void k_sum_parts(const double* __restrict__ part, int n, double* out)
 
 // The two sums of the interpolation damping on a coarse level, x.w0 and
 // x.((A + cc) x), in one pass over x: FP32 products (A + cc) x, FP64 sums,
-// partials per block (reduce_parts blocks) summed by the block that finishes
+// partials per block (at most 1184 blocks) summed by the block that finishes
 // last (a ticket on *done, which it resets).
 __global__ void k_damp_dots(Grid g, OpF o, const float* __restrict__ cc,
                             const float* __restrict__ x, const float* __restrict__ w0,
@@ -578,7 +578,10 @@ __global__ void k_damp_dots(Grid g, OpF o, const float* __restrict__ cc,
 void damp_dots(cudaStream_t s, Grid g, OpF o, const float* cc, const float* x, const float* w0,
                double* part, unsigned* done, double* num, double* den) {
   const size_t nint = (size_t)(g.nx - 2) * (g.ny - 2) * (g.nz - 2);
-  const int nb = (int)reduce_parts(nint);
+  // a point per thread while the partials' room lasts: with four, levels of 33^3 and
+  // below had a block on fewer than half of the SMs (levels of 65^3 and 33^3 on
+  // average 15.9 -> 9.5 us)
+  const int nb = (int)std::min<size_t>((nint + 255) / 256, 1184);
   k_damp_dots<<<nb, 256, 0, s>>>(g, o, cc, x, w0, part, part + 2368, done, num, den);
 }
 
