@@ -952,8 +952,8 @@ int launch_gs27_planes(cudaStream_t s, Grid g, Op op, const double* cc, const do
 //    for a pass that needs no order.
 // Measured (two sweeps and the residual; in brackets the kernels before, whole
 // planes in shared memory and a global mailbox, at 113^3 step counters):
-// 17^3 40 us (66), 33^3 68 (126), 49^3 99 (203), 65^3 137 (289), 81^3 222 (455),
-// 97^3 296 (744), 113^3 399 (1244).  One group of threads for all rows of a
+// 17^3 40 us (66), 33^3 68 (126), 49^3 98 (203), 65^3 135 (289), 81^3 215 (455),
+// 97^3 286 (744), 113^3 387 (1244).  One group of threads for all rows of a
 // half-sweep: 81^3 300, 49^3 150.
 //
 // Why a neighbour stays within wlag rows: half-sweep q of the lower plane can
