@@ -947,7 +947,8 @@ int launch_gs27_planes(cudaStream_t s, Grid g, Op op, const double* cc, const do
 //  * A quotient by the prefetched reciprocal, correctly rounded (div_by).
 //  * At the edge of a cluster, couriers (two warps) poll the foreign
 //    neighbour's global slots, two rows at a time, and put the values into the
-//    inbox: the polls' round trips are off the workers' path.
+//    inbox: the polls' round trips are off the workers' path.  Any cluster size
+//    works, one CTA included (tests/test_gs27_mail_clusters.py).
 //  * The residual is a kernel of its own: it would double the loads of a step
 //    for a pass that needs no order.
 // Measured (two sweeps and the residual; in brackets the kernels before, whole
@@ -1284,60 +1285,72 @@ __global__ void __launch_bounds__(2 * kMailHalfMax * mail_width(HP) + kMailHelpe
       }
     }
   } else if ((int)threadIdx.x >= nwork) {
-    // ---- couriers: the foreign neighbour's global slots into the inbox
-    const int side = (rank == 0 && c > 0) ? 0 : ((rank == clsize - 1 && c + 1 < ncta) ? 1 : -1);
+    // ---- couriers: the foreign neighbours' global slots into the inbox, the lower
+    // plane's (side 0) where the cluster begins here, the upper one's (side 1) where it
+    // ends here.  Both in a cluster of one CTA: no plan asks for that, but a kernel
+    // must not hang on the cluster it arrives with.
+    const bool foreign[2] = {rank == 0 && c > 0, rank == clsize - 1 && c + 1 < ncta};
     const int u = threadIdx.x - nwork;
-    const int nslot = side < 0 ? 0 : (side == 0 ? nhalf : nhalf - 1) * hr;
-    const int cn = side == 0 ? c - 1 : c + 1, kn = 1 + cn;
     constexpr int kSlots = (kMailHalfMax * HP + kMailCouriers - 1) / kMailCouriers;
-    int row[kSlots], q[kSlots], m[kSlots];
+    int row[2][kSlots], q[kSlots], m[kSlots];
 #pragma unroll
     for (int n = 0; n < kSlots; n++) {
       q[n] = (u + n * kMailCouriers) / hr;
       m[n] = u + n * kMailCouriers - q[n] * hr;
     }
     // the first row from r on whose colour has this slot (odd nx: the last
-    // slot exists on every other row)
+    // slot exists on every other row; k - 1 and k + 1 have the same parity)
     auto valid_from = [&](int n, int r) -> int {
-      const int b = (((1 + r + kn) & 1) != ((first_parity + q[n]) & 1)) ? 1 : 0;
+      const int b = (((r + k) & 1) != ((first_parity + q[n]) & 1)) ? 1 : 0;
       return (1 + b + 2 * m[n] <= nx - 2) ? r : r + 1;
     };
 #pragma unroll
-    for (int n = 0; n < kSlots; n++)
-      row[n] = u + n * kMailCouriers < nslot ? valid_from(n, 1) : ny;
+    for (int side = 0; side < 2; side++)
+#pragma unroll
+      for (int n = 0; n < kSlots; n++)
+        row[side][n] = foreign[side] && u + n * kMailCouriers < (nhalf - side) * hr
+                           ? valid_from(n, 1)
+                           : ny;
     unsigned long long t0 = 0;
     for (int spins = 1;; spins++) {
-      unsigned long long w[kSlots][2][2];
-      int nrow[kSlots];
       bool left = false;
 #pragma unroll
-      for (int n = 0; n < kSlots; n++) {
-        nrow[n] = ny;
-        if (row[n] > ny - 2) continue;
-        left = true;
-        nrow[n] = valid_from(n, row[n] + 1);
-        const unsigned long long* p0 =
-            mail + 2 * ((((ptrdiff_t)cn * nhalf + q[n]) * (ny - 2) - 1) * hr + m[n]);
-        mail_load(p0 + 2 * (size_t)row[n] * hr, w[n][0][0], w[n][0][1]);
-        if (nrow[n] <= ny - 2) mail_load(p0 + 2 * (size_t)nrow[n] * hr, w[n][1][0], w[n][1][1]);
-      }
-      if (!left) break;
+      for (int side = 0; side < 2; side++) {
+        if (!foreign[side]) continue;
+        const ptrdiff_t cn = side == 0 ? c - 1 : c + 1;
+        unsigned long long w[kSlots][2][2];
+        int nrow[kSlots];
 #pragma unroll
-      for (int n = 0; n < kSlots; n++) {
+        for (int n = 0; n < kSlots; n++) {
+          int& at = row[side][n];
+          nrow[n] = ny;
+          if (at > ny - 2) continue;
+          left = true;
+          nrow[n] = valid_from(n, at + 1);
+          const unsigned long long* p0 =
+              mail + 2 * (((cn * nhalf + q[n]) * (ny - 2) - 1) * hr + m[n]);
+          mail_load(p0 + 2 * (size_t)at * hr, w[n][0][0], w[n][0][1]);
+          if (nrow[n] <= ny - 2) mail_load(p0 + 2 * (size_t)nrow[n] * hr, w[n][1][0], w[n][1][1]);
+        }
 #pragma unroll
-        for (int d = 0; d < 2; d++) {
-          if (row[n] > ny - 2 || (d == 1 && row[n] != nrow[n])) break;
-          if (!mail_is(w[n][d][0], w[n][d][1], tag)) break;
-          const unsigned long long it =
-              (unsigned long long)(itag0 + (unsigned)row[n] / kMailInRows) << 32;
-          unsigned long long* s = inbox + (side * kMailHalfMax + q[n]) * IBOX +
-                                  (row[n] % kMailInRows) * IROW + 2 * m[n];
-          inbox_put((unsigned)__cvta_generic_to_shared(s), (w[n][d][0] & 0xffffffffull) | it,
-                    (w[n][d][1] & 0xffffffffull) | it);
-          row[n] = d == 0 ? nrow[n] : valid_from(n, row[n] + 1);
-          t0 = 0;
+        for (int n = 0; n < kSlots; n++) {
+          int& at = row[side][n];
+#pragma unroll
+          for (int d = 0; d < 2; d++) {
+            if (at > ny - 2 || (d == 1 && at != nrow[n])) break;
+            if (!mail_is(w[n][d][0], w[n][d][1], tag)) break;
+            const unsigned long long it =
+                (unsigned long long)(itag0 + (unsigned)at / kMailInRows) << 32;
+            unsigned long long* s = inbox + (side * kMailHalfMax + q[n]) * IBOX +
+                                    (at % kMailInRows) * IROW + 2 * m[n];
+            inbox_put((unsigned)__cvta_generic_to_shared(s), (w[n][d][0] & 0xffffffffull) | it,
+                      (w[n][d][1] & 0xffffffffull) | it);
+            at = d == 0 ? nrow[n] : valid_from(n, at + 1);
+            t0 = 0;
+          }
         }
       }
+      if (!left) break;
       if ((spins & 63) == 0 && !keep_waiting(t0)) break;
     }
   } else {
@@ -1596,11 +1609,12 @@ int wave_mail_fit(Grid g) { return mail_plan(g, kMailHalfMax).kernel != nullptr;
 
 int launch_gs27_mail(cudaStream_t s, Grid g, const double* pack, const double* fc, double* x,
                      int x_zero, int nsweep, int first_parity, unsigned* counters, int* err,
-                     int wlag, unsigned long long* mail) {
+                     int wlag, unsigned long long* mail, int cluster) {
   const int nhalf = 2 * nsweep;
   if (!mail || !pack) return 0;
-  const MailPlan p = mail_plan(g, nhalf);
+  MailPlan p = mail_plan(g, nhalf);
   if (!p.kernel) return 0;
+  if (cluster > 0) p.cluster = cluster;
   wlag = wlag < 6 ? std::max(wlag, 4) : mail_lag(pack_hr(g));
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((g.nz - 2 + p.cluster - 1) / p.cluster * p.cluster, 1, 1);

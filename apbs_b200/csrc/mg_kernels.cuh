@@ -73,6 +73,7 @@ int launch_gs27_wave(cudaStream_t s, Grid g, Op op, const double* cc, const doub
 // 64-bit words per level, zeroed whenever the level's counters restart), from
 // the packed coefficients of launch_gs27_pack (gs27_pack_doubles(g) doubles).
 // x_zero: x is taken as zero whatever it holds (its boundary has to be).
+// cluster: CTAs per cluster, 0 for the plan's (the iterates do not depend on it).
 // wave_mail_fit: a row's points fit the CTA's threads and the level's planes
 // the device.  Returns 0 (nothing launched) where it does not fit.
 size_t mail_words(Grid g);
@@ -82,7 +83,7 @@ int wave_mail_fit(Grid g);
 void launch_gs27_pack(cudaStream_t s, Grid g, Op op, const double* cc, double* pack, int coef);
 int launch_gs27_mail(cudaStream_t s, Grid g, const double* pack, const double* fc, double* x,
                      int x_zero, int nsweep, int first_parity, unsigned* counters, int* err,
-                     int wlag, unsigned long long* mail);
+                     int wlag, unsigned long long* mail, int cluster);
 
 // ---- BLAS-1 on interior points -------------------------------------------
 void launch_zero(cudaStream_t s, double* x, size_t n);

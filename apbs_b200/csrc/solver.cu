@@ -1062,7 +1062,7 @@ static int gs27_smooth(pmgb_solver* s, cudaStream_t st, int l, const double* cc,
       launch_gs27_mail(st, L.g, s->d_pack + s->pack_off[l], fc, x, x_zero, 2, first_parity,
                        s->d_wave + kWaveCounterBase + (size_t)l * kWavePlanesMax,
                        reinterpret_cast<int*>(s->d_wave), s->tune[PMGB_TUNE_GS27_LAG],
-                       s->d_mail + s->mail_off[l])) {
+                       s->d_mail + s->mail_off[l], s->mail_cluster)) {
     s->wave_used = 1;
     k++;
     if (r) {
@@ -1398,6 +1398,24 @@ extern "C" int pmgb_debug_shift_wave_counter(pmgb_solver* s, int level, int plan
   CK(cudaMemcpy(&v, c, sizeof(v), cudaMemcpyDeviceToHost));
   v += (unsigned)delta;
   CK(cudaMemcpy(c, &v, sizeof(v), cudaMemcpyHostToDevice));
+  return 1;
+}
+
+// Testing hook: the mailbox wavefront of this calculation in clusters of that
+// many CTAs (0: its plan's choice); the iterates do not depend on it.
+extern "C" int pmgb_debug_wave_cluster(pmgb_solver* s, int cluster) {
+  if (!s || (cluster != 0 && cluster != 1 && cluster != 2 && cluster != 4 && cluster != 8 &&
+             cluster != 16)) {
+    set_error("pmgb_debug_wave_cluster: the cluster must be 0, 1, 2, 4, 8 or 16");
+    return 0;
+  }
+  CK(cudaStreamSynchronize(s->stream));
+  s->mail_cluster = cluster;
+  for (int m = 0; m < 2; m++)  // the captured V-cycles hold the launch's shape
+    if (s->vc_exec[m]) {
+      cudaGraphExecDestroy(s->vc_exec[m]);
+      s->vc_exec[m] = nullptr;
+    }
   return 1;
 }
 

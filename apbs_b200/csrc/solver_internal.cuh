@@ -142,6 +142,7 @@ struct pmgb_solver {
   unsigned long long* d_mail;
   long long mail_off[12];
   size_t mail_total;
+  int mail_cluster;  // CTAs per cluster of the mailbox wavefront, 0: its plan's (testing hook)
   // FP64 only: packed coefficients of the same levels (launch_gs27_pack);
   // pack_cc: the Helmholtz terms their diagonals hold (0 none yet, 1 cc, 2 cp)
   double* d_pack;

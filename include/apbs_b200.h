@@ -136,6 +136,11 @@ int pmgb_forces(pmgb_solver *s, double *qf, double *db, double *ib);
  * after it runs normally.  No reference counterpart. */
 int pmgb_debug_shift_wave_counter(pmgb_solver *s, int level, int plane, int delta);
 
+/* Testing hook: the plane-parallel GS27 wavefront of this calculation in
+ * clusters of 1, 2, 4, 8 or 16 CTAs (0: the size its plan picks).  The
+ * iterates do not depend on it.  No reference counterpart. */
+int pmgb_debug_wave_cluster(pmgb_solver *s, int cluster);
+
 /* OpenDX output, byte for byte the file writedataMG writes through
  * Vgrid_writeDX (src/routines.c:2620-2920, src/mg/vgrid.c:1206-1420):
  * pmgb_write_dx writes one map of a calculation with its partition weights
