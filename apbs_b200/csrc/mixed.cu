@@ -845,7 +845,9 @@ __device__ __forceinline__ void tail_sync() {
 
 // Sum of two values over the cluster, the same result in every thread.  Each CTA
 // stores its partial sums into every CTA's slots ahead of the barrier, so after it
-// they are read locally, in rank order.  slots: [2 phases][CLUSTER][2].
+// they are read locally, in rank order.  slots: [2 phases][CLUSTER][2].  A CTA may
+// store into another's shared memory only once that one is known to run: every
+// kernel passes a tail_sync before its first sum (tests/test_cluster_first_push.py).
 template <int CLUSTER>
 __device__ void tail_sum2(double& a, double& b, double* sh, double* slots, int& phase) {
   a = warp_sum(a);
@@ -1348,6 +1350,7 @@ __global__ void __launch_bounds__(512) k_batch_solve(const BatchItem* __restrict
   const BatchItem& B = *reinterpret_cast<const BatchItem*>(item);
   TailArgs T = B.T;
   tail_levels(T, levels);
+  tail_sync<CLUSTER>();  // every CTA runs before the first sum stores into its slots
   const TailTid tid = tail_tid<CLUSTER>();
   int phase = 0;
   const Grid g = B.g;
