@@ -782,18 +782,21 @@ __device__ __forceinline__ float nb27t(const TLev& L, const float* x, size_t id)
   return nb27(o, L.g, x, id);
 }
 
-// q / d by multiplication with div_const(d) = ceil(2^32 / d) (0: d = 1): exact for
-// q < 2^32 / d, which the levels of one cluster are far below.
+// q / d for 0 <= q < 2^31 by multiplication with c = div_const(d) = ceil(2^32 / d)
+// (0: d = 1): q c / 2^32 is q / d plus less than 1/2, so its whole part is the
+// quotient or one more (tests/test_long_axes.py).
 inline unsigned div_const(int d) {
   return d > 1 ? (unsigned)((0x100000000ull + d - 1) / d) : 0u;
 }
-__device__ __forceinline__ int quotient(int q, unsigned c) {
-  return c ? (int)__umulhi((unsigned)q, c) : q;
+__device__ __forceinline__ int quotient(int q, int d, unsigned c) {
+  if (!c) return q;
+  const unsigned t = __umulhi((unsigned)q, c);
+  return (int)(t - (t * (unsigned)d > (unsigned)q ? 1u : 0u));
 }
 // Interior point q of a level as a flat index.
 __device__ __forceinline__ int interior_at(Grid g, unsigned dx, unsigned dy, int q) {
   const int ex = g.nx - 2, ey = g.ny - 2;
-  const int t = quotient(q, dx), k = quotient(t, dy);
+  const int t = quotient(q, ex, dx), k = quotient(t, ey, dy);
   return ((k + 1) * g.ny + t - k * ey + 1) * g.nx + q - t * ex + 1;
 }
 
@@ -1016,15 +1019,15 @@ __device__ void tail_damp(const TLev& L, TailTid tid, double* sh, double* slots,
 __device__ void tail_interp(Grid gc, const float* xc, Grid gf, unsigned dx, unsigned dy, float* xf,
                             float xdamp, TailTid tid) {
   const int ex = gf.nx - 2, ey = gf.ny - 2, nint = ex * ey * (gf.nz - 2);
+  struct Corrected {
+    int id;
+    float x;
+  };
   for_points<2>(
-      nint, tid,
+      nint, tid, [](int q) { return q; },
       [&](int q) {
-        const int t = quotient(q, dx), k = quotient(t, dy);
-        // packed (i, j, k): 10 bits each hold the points of a cluster's levels
-        return (q - t * ex + 1) | (t - k * ey + 1) << 10 | (k + 1) << 20;
-      },
-      [&](int ijk) {
-        const int i = ijk & 1023, j = (ijk >> 10) & 1023, k = ijk >> 20;
+        const int t = quotient(q, ex, dx), k = quotient(t, ey, dy) + 1;
+        const int i = q - t * ex + 1, j = t - (k - 1) * ey + 1;
         const int ii = i >> 1, jj = j >> 1, kk = k >> 1;
         const int oi = i & 1, oj = j & 1, ok = k & 1;
         float w = 0.f;
@@ -1032,11 +1035,10 @@ __device__ void tail_interp(Grid gc, const float* xc, Grid gf, unsigned dx, unsi
           for (int b = 0; b <= oj; b++)
             for (int a = 0; a <= oi; a++) w += xc[gc.idx(ii + a, jj + b, kk + c)];
         w *= 1.f / (float)(1 << (oi + oj + ok));
-        return make_float2(w, xf[gf.idx(i, j, k)]);
+        const int id = (k * gf.ny + j) * gf.nx + i;
+        return Corrected{id, xf[id] + xdamp * w};
       },
-      [&](int ijk, float2 v) {
-        xf[gf.idx(ijk & 1023, (ijk >> 10) & 1023, ijk >> 20)] = v.y + xdamp * v.x;
-      });
+      [&](int, Corrected v) { xf[v.id] = v.x; });
 }
 
 // The level table in shared memory (kTailLevels at most): the pointers of a pass
@@ -1316,7 +1318,7 @@ __device__ void batch_gs7(const BatchItem& B, unsigned dh, unsigned dy, int pari
   for_points<4>(
       nslots, tid,
       [&](int q) {
-        const int t = quotient(q, dh), k = quotient(t, dy) + 1;
+        const int t = quotient(q, hr, dh), k = quotient(t, ey, dy) + 1;
         const int m = q - t * hr, j = t - (k - 1) * ey + 1;
         const int off = ((1 + j + k) & 1) != parity;
         const int i = 1 + off + 2 * m;
