@@ -19,6 +19,7 @@
 // 25 us against 0.88 ms.  The factors take 6.7 ms at 27^3, 1.7 ms at 19^3 and
 // 0.52 ms at 11^3, once per operator.
 #include <algorithm>
+#include <mutex>
 
 #include "coarse_direct.cuh"
 #include "mixed.cuh"
@@ -466,19 +467,39 @@ __global__ void __launch_bounds__(kSolveThreads, 1) k_direct_solve(Args A) {
   if (tid == 0) A.counters[blockIdx.x] = tag;
 }
 
-size_t factor_smem(int pp) { return 2 * (size_t)kRows * pp * sizeof(double); }
-size_t solve_smem(int pp) {
+constexpr size_t factor_smem(int pp) { return 2 * (size_t)kRows * pp * sizeof(double); }
+constexpr size_t solve_smem(int pp) {
   return (2 * (size_t)kRows * pp + 2 * (size_t)pp + kPlanesMax * kRows) * sizeof(double);
 }
+// The largest plane: its slabs (two in the solve) and the static arrays in a
+// CTA's 227 KB of shared memory.
+constexpr int kPlaneMax = 816;
+static_assert(factor_smem(kPlaneMax) + 16384 <= 232448 && solve_smem(kPlaneMax) + 1024 <= 232448 &&
+                  solve_smem(kPlaneMax + kRows) + 1024 > 232448 && kPlaneMax <= 2 * kSolveThreads,
+              "kPlaneMax");
 
-// Unknowns of a plane in whole blocks, 0 where the level does not fit: a
-// plane's rows in two CTAs' worth of SMs, two slabs of them in shared memory.
+// Unknowns of a plane in whole blocks, 0 where the level does not fit.
 int direct_blocks(Grid g) {
   const int p = (g.nx - 2) * (g.ny - 2), ez = g.nz - 2;
   const int pp = (p + kRows - 1) / kRows * kRows;
-  if (ez > kPlanesMax || p > 2 * kSolveThreads) return 0;
-  if (factor_smem(pp) + 16384 > 232448 || solve_smem(pp) + 1024 > 232448) return 0;
-  return pp;
+  return ez <= kPlanesMax && pp <= kPlaneMax ? pp : 0;
+}
+
+// The kernels' limits of dynamic shared memory belong to the process, not to a
+// calculation: set once per device, to what the largest plane takes.  (A
+// calculation that set its own would lower the limit under one with larger
+// planes, whose next launches were refused.)
+bool direct_smem_ready(int dev) {
+  static std::once_flag once[16];
+  static bool ok[16];
+  if (dev < 0 || dev >= 16) return false;
+  std::call_once(once[dev], [dev] {
+    ok[dev] = cudaFuncSetAttribute(k_direct_factor, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   (int)factor_smem(kPlaneMax)) == cudaSuccess &&
+              cudaFuncSetAttribute(k_direct_solve, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   (int)solve_smem(kPlaneMax)) == cudaSuccess;
+  });
+  return ok[dev];
 }
 
 }  // namespace
@@ -519,10 +540,7 @@ static int direct_alloc(pmgb_solver* s, Grid g, int pp) {
   cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
   const int ctas = 2 * (pp / kRows);
   if (!coop || ctas > sms) return 0;
-  if (cudaFuncSetAttribute(k_direct_factor, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)factor_smem(pp)) != cudaSuccess ||
-      cudaFuncSetAttribute(k_direct_solve, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)solve_smem(pp)) != cudaSuccess ||
+  if (!direct_smem_ready(dev) ||
       cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_direct_factor, kFactorThreads,
                                                     factor_smem(pp)) != cudaSuccess ||
       per * sms < ctas ||
