@@ -22,6 +22,7 @@
 #include <mutex>
 
 #include "coarse_direct.cuh"
+#include "mg_kernels.cuh"
 #include "mixed.cuh"
 #include "solver_internal.cuh"
 
@@ -593,7 +594,7 @@ static Args direct_args(pmgb_solver* s) {
   A.piv = d->piv;
   A.flag = d->words;
   A.info = d->info;
-  A.err = reinterpret_cast<int*>(s->d_wave);
+  A.err = reinterpret_cast<int*>(s->d_wave) + kWaveDirectErr;
   A.b = nullptr;
   A.x = nullptr;
   A.mail = d->mail;
@@ -622,10 +623,16 @@ int direct_prepare(pmgb_solver* s) {
     return 0;
   }
   note_launches(2);
-  s->wave_used = 1;  // its waits are counted with the wavefronts'
-  int info[2] = {0, 0};
+  s->wave_used = 1;  // the solve's waits are looked at where the wavefronts' are
+  int info[2] = {0, 0}, nerr = 0;
   PMGB_CUDA_OK(cudaMemcpyAsync(info, d->info, sizeof(info), cudaMemcpyDeviceToHost, st));
+  PMGB_CUDA_OK(cudaMemcpyAsync(&nerr, A.err, sizeof(int), cudaMemcpyDeviceToHost, st));
   PMGB_CUDA_OK(cudaStreamSynchronize(st));
+  if (nerr) {  // the factors are not whole: no later solve may take them
+    PMGB_CUDA_OK(cudaMemsetAsync(A.err, 0, sizeof(int), st));
+    set_error("%d bounded device waits ran out (factor of the direct coarse solve)", nerr);
+    return -1;
+  }
   // a pivot that is not positive, or a band entry that is no grid neighbour's:
   // the band factor decides
   return info[0] == 0 && info[1] == 0;

@@ -193,19 +193,24 @@ float elapsed_ms(cudaEvent_t a, cudaEvent_t b) {
   return ms;
 }
 
+// The counts of bounded waits that ran out, d_wave's first words: 1 if none
+// did, else the error that names their kernels.
+int waits_held(const int* nerr) {
+  static_assert(kWaveDirectErr == 1, "the counts are read together");
+  if (nerr[0]) set_error("%d bounded device waits ran out (gs27 plane wavefront)", nerr[0]);
+  else if (nerr[1]) set_error("%d bounded device waits ran out (direct coarse solve)", nerr[1]);
+  return !nerr[0] && !nerr[1];
+}
+
 int read_scalar(pmgb_solver* s, int slot, double* v) {
   CK(cudaMemcpyAsync(v, s->scal + slot, sizeof(double), cudaMemcpyDeviceToHost, s->stream));
-  // a plane-wavefront wait that ran out leaves the iterates undefined: stop
-  // at the next read instead of iterating on them (pmgb_solve reports it)
-  int nerr = 0;
+  // a wait that ran out leaves the iterates undefined: stop at the next read
+  // instead of iterating on them (pmgb_solve reports it)
+  int nerr[2] = {0, 0};
   if (s->wave_used)
-    CK(cudaMemcpyAsync(&nerr, s->d_wave, sizeof(int), cudaMemcpyDeviceToHost, s->stream));
+    CK(cudaMemcpyAsync(nerr, s->d_wave, sizeof(nerr), cudaMemcpyDeviceToHost, s->stream));
   CK(cudaStreamSynchronize(s->stream));
-  if (nerr) {
-    set_error("%d bounded device waits ran out (gs27 plane wavefront)", nerr);
-    return 0;
-  }
-  return 1;
+  return waits_held(nerr);
 }
 
 // GS27 launch shape per level (cluster of CTAs for the wavefront).
@@ -998,7 +1003,9 @@ static int build_ops(pmgb_solver* s) {
     // factor and its substitutions are sequential
     const Grid gc = s->lev[s->nlev - 1].g;
     if ((size_t)(gc.nx - 2) * (gc.ny - 2) * (gc.nz - 2) > 512 && s->tune[4] == 0) {
-      if (direct_prepare(s)) s->mgsolv = 3;
+      const int direct = direct_prepare(s);
+      if (direct < 0) return 0;
+      if (direct) s->mgsolv = 3;
       else if (coarse_exact_prepare(s)) s->mgsolv = 2;
     }
   }
@@ -1367,22 +1374,32 @@ int pmgb::newton_driver(pmgb_solver* s, double errtol, int itmax, int mixed) {
   return 1;
 }
 
-// Reads (and clears) the count of plane-wavefront waits that ran out; a
-// nonzero count fails the solve (the iterates are not the ordered sweep's).
+// Reads (and clears) the counts of plane-wavefront and direct-solve waits that
+// ran out; a nonzero count fails the solve (the iterates are undefined).
 static int wave_check(pmgb_solver* s) {
   // wave_used stays set: graphs captured with the plane kernel replay it in
   // every later solve without passing through gs27_smooth again
   if (!s->wave_used) return 1;
-  int nerr = 0;
-  CK(cudaMemcpyAsync(&nerr, s->d_wave, sizeof(int), cudaMemcpyDeviceToHost, s->stream));
+  int nerr[2] = {0, 0};
+  CK(cudaMemcpyAsync(nerr, s->d_wave, sizeof(nerr), cudaMemcpyDeviceToHost, s->stream));
   CK(cudaStreamSynchronize(s->stream));
-  if (nerr) {
+  if (!waits_held(nerr)) {
     // the counters of the levels may now disagree: restart them all
     wave_reset(s, s->stream);
     CK(cudaStreamSynchronize(s->stream));
-    set_error("%d bounded device waits ran out (gs27 plane wavefront)", nerr);
     return 0;
   }
+  return 1;
+}
+
+// Testing hook: count a wait of the direct coarse solve as run out.
+extern "C" int pmgb_debug_direct_wait(pmgb_solver* s) {
+  if (!s) {
+    set_error("pmgb_debug_direct_wait: no calculation");
+    return 0;
+  }
+  const int one = 1;
+  CK(cudaMemcpy(s->d_wave + kWaveDirectErr, &one, sizeof(one), cudaMemcpyHostToDevice));
   return 1;
 }
 

@@ -127,13 +127,13 @@ struct pmgb_solver {
   int nref;
   size_t ref_alloc;
   int* d_npts;
-  // step counters of the plane-parallel GS27 wavefront: word 0 counts waits
-  // that ran out, level l's counters start at kWaveCounterBase + l *
-  // kWavePlanesMax
   UserMap maps[PMGB_MAP_COUNT];  // usemap diel/kappa/charge
   double* map_scratch;      // kappa-map maximum and error counts
   double* d_forces;         // pmgb_forces: 9 doubles and a status word per atom
   size_t forces_alloc;
+  // step counters of the plane-parallel GS27 wavefront: word 0 counts its waits
+  // that ran out, word kWaveDirectErr those of the direct coarse solve, level l's
+  // counters start at kWaveCounterBase + l * kWavePlanesMax
   unsigned* d_wave;
   int wave_used;  // the plane kernel has been launched or captured (stays set)
   // mailboxes of the shared-memory plane wavefront: level l's starts at word

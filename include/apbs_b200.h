@@ -136,6 +136,13 @@ int pmgb_forces(pmgb_solver *s, double *qf, double *db, double *ib);
  * after it runs normally.  No reference counterpart. */
 int pmgb_debug_shift_wave_counter(pmgb_solver *s, int level, int plane, int delta);
 
+/* Testing hook for the failure path of the direct coarse solve (FP64 LPBE):
+ * counts one of its bounded waits as run out, so that the factor in the next
+ * build, or else the next coarse solve, gives up its waits (no device fault).
+ * That pmgb_solve fails with an error naming the waits; the one after it makes
+ * the factors again where they were not whole.  No reference counterpart. */
+int pmgb_debug_direct_wait(pmgb_solver *s);
+
 /* Testing hook: the plane-parallel GS27 wavefront of this calculation in
  * clusters of 1, 2, 4, 8 or 16 CTAs (0: the size its plan picks).  The
  * iterates do not depend on it.  No reference counterpart. */
