@@ -24,6 +24,7 @@
 #include "coarse_direct.cuh"
 #include "mg_kernels.cuh"
 #include "mixed.cuh"
+#include "quotients.cuh"
 #include "solver_internal.cuh"
 
 namespace pmgb {
@@ -114,16 +115,6 @@ __device__ __forceinline__ double in_plane(const Args& A, int i, int j, int ci, 
   // a diagonal neighbour: stored at the lower row's point, to the east or west
   if (dy > 0) return -A.op[dx > 0 ? ONE : ONW][A.g.idx(i, j, k)];
   return -A.op[dx < 0 ? ONE : ONW][A.g.idx(ci, cj, k)];
-}
-
-// 1 / x by Newton's iteration on the hardware's 20-bit approximation: two steps
-// reach 80 bits in exact arithmetic
-__device__ __forceinline__ double reciprocal(double x) {
-  double y;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  y = fma(fma(-x, y, 1.0), y, y);
-  y = fma(fma(-x, y, 1.0), y, y);
-  return fma(fma(-x, y, 1.0), y, y);
 }
 
 // The inverses D_k.  One CTA per 16 rows of a plane's matrix and side, its rows
@@ -503,6 +494,15 @@ bool direct_smem_ready(int dev) {
   return ok[dev];
 }
 
+// The quotients of quotients.cuh beside the division's, for the test.
+__global__ void k_quotients(int n, const double* a, const double* b, double* out) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  out[i] = a[i] / b[i];
+  out[n + i] = div_by(a[i], b[i], div_factor(b[i]));
+  out[2 * n + i] = reciprocal(b[i]);
+}
+
 }  // namespace
 
 struct DirectState {
@@ -653,3 +653,24 @@ int launch_direct_solve(pmgb_solver* s, cudaStream_t st, const double* b, double
 }
 
 }  // namespace pmgb
+
+// Testing hook: a / b by division and by div_by, and reciprocal(b), of n pairs; out
+// has 3 n values.
+extern "C" int pmgb_debug_quotients(int n, const double* a, const double* b, double* out) {
+  using namespace pmgb;
+  if (n < 1 || n > (1 << 24) || !a || !b || !out) {
+    set_error("pmgb_debug_quotients: bad arguments");
+    return 0;
+  }
+  const size_t bytes = (size_t)n * sizeof(double);
+  double* d = nullptr;
+  PMGB_CUDA_OK(cudaMalloc((void**)&d, 5 * bytes));
+  cudaMemcpy(d, a, bytes, cudaMemcpyHostToDevice);
+  cudaMemcpy(d + n, b, bytes, cudaMemcpyHostToDevice);
+  k_quotients<<<(n + 255) / 256, 256>>>(n, d, d + n, d + 2 * (size_t)n);
+  note_launches(1);
+  const cudaError_t e = cudaMemcpy(out, d + 2 * (size_t)n, 3 * bytes, cudaMemcpyDeviceToHost);
+  cudaFree(d);
+  PMGB_CUDA_OK(e);
+  return 1;
+}

@@ -13,6 +13,7 @@
 
 #include "gs7_rb.cuh"
 #include "mg_kernels.cuh"
+#include "quotients.cuh"
 
 namespace cg = cooperative_groups;
 
@@ -933,7 +934,8 @@ int launch_gs27_planes(cudaStream_t s, Grid g, Op op, const double* cc, const do
 //    of a row's instructions, of which the late part is a third.
 //  * Coefficients in the order an update reads them (k_gs27_pack): per row and
 //    colour, 14 pairs of doubles for each point, contiguous over the points of
-//    the colour -- the 26 couplings, the diagonal D = oC + cc and 1/D.  Read
+//    the colour -- the 26 couplings, the diagonal D = oC + cc and its factor
+//    (div_factor).  Read
 //    from the 14 operator arrays a colour uses half of each sector and 28
 //    address computations per point.  A warp of its own brings them in by bulk
 //    copies, which take no part of the load pipe the workers' critical loads
@@ -1004,20 +1006,6 @@ __device__ __forceinline__ void mail_load(const unsigned long long* p, unsigned 
                                           unsigned long long& w1) {
   asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(w0), "=l"(w1) : "l"(p));
 }
-// a / b with y = RN(1/b): P. Markstein's quotient (IBM J. Res. Dev. 34, 1990):
-// with y correctly rounded, a quotient within one ulp of a / b is corrected
-// to the rounded one by its exact remainder times y; the first correction
-// brings a*y (up to 1.5 ulp off) there.  Outside the range where a remainder
-// could underflow or overflow, the division itself.
-__device__ __forceinline__ double div_by(double a, double b, double y) {
-  const double q0 = a * y;
-  const double q1 = __fma_rn(__fma_rn(-b, q0, a), y, q0);
-  const double q2 = __fma_rn(__fma_rn(-b, q1, a), y, q1);
-  const unsigned e = (unsigned)__double2hiint(q0) & 0x7fffffffu;  // exponent of the quotient
-  if (e - 0x10000000u < 0x60000000u || a == 0.0) return q2;       // 2^-767 .. 2^769, or 0 / b
-  return a / b;
-}
-
 static int mail_hr(Grid g) { return (g.nx - 1) / 2; }         // points of one colour in a row
 static int pack_hr(Grid g) { return (mail_hr(g) + 7) & ~7; }  // the same, in whole lines
 
@@ -1056,7 +1044,7 @@ __global__ void k_gs27_pack(Grid g, Op op, const double* __restrict__ cc, double
     }
     const size_t id = g.idx(i, j, k);
     const double d = op.c[OC][id] + cc[id];
-    out[(size_t)13 * hp] = make_double2(d, 1.0 / d);
+    out[(size_t)13 * hp] = make_double2(d, div_factor(d));
     if (!coef) continue;
     Coef27 C;
     load_coef27(op, cc, cc, id, sy, sz, C);

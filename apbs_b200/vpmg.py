@@ -94,6 +94,7 @@ def lib():
         L.pmgb_forces.argtypes = [vp, dp, dp, dp]
         L.pmgb_debug_shift_wave_counter.argtypes = [vp, ctypes.c_int, ctypes.c_int, ctypes.c_int]
         L.pmgb_debug_direct_wait.argtypes = [vp]
+        L.pmgb_debug_quotients.argtypes = [ctypes.c_int, dp, dp, dp]
         L.pmgb_debug_wave_cluster.argtypes = [vp, ctypes.c_int]
         L.pmgb_write_dx.argtypes = [vp, ctypes.c_int, ctypes.c_char_p, ctypes.c_char_p,
                                     ctypes.c_char_p]

@@ -143,6 +143,11 @@ int pmgb_debug_shift_wave_counter(pmgb_solver *s, int level, int plane, int delt
  * the factors again where they were not whole.  No reference counterpart. */
 int pmgb_debug_direct_wait(pmgb_solver *s);
 
+/* Testing hook: of n pairs of host values a[i], b[i], the quotients by division
+ * and by the wavefront's multiplication, and the plane factor's reciprocal of
+ * b[i] (out: n values of each).  No reference counterpart. */
+int pmgb_debug_quotients(int n, const double *a, const double *b, double *out);
+
 /* Testing hook: the plane-parallel GS27 wavefront of this calculation in
  * clusters of 1, 2, 4, 8 or 16 CTAs (0: the size its plan picks).  The
  * iterates do not depend on it.  No reference counterpart. */
