@@ -1543,6 +1543,13 @@ Gs7Rb<float> rb_f32(const MLevel& F, const float* d32, const int* tune) {
 // bits.  k counts the kernels launched.
 constexpr size_t kSinglePassMin = 3000000;
 
+bool gs7_f32_single(Grid g, const int* tune) {
+  const size_t fint = (size_t)(g.nx - 2) * (g.ny - 2) * (g.nz - 2);
+  return tune[5] == 2 ? (g.nx & 1) && (g.ny & 1)
+                      : tune[5] == 0 && fint >= kSinglePassMin &&
+                            gs7_rb_suits<float>(g.nx, g.ny, g.n(), tune[12]);
+}
+
 cudaError_t gs7_f32(cudaStream_t st, const MLevel& F, float* x, float* r, int first_parity,
                     float* xs, const float* d32, bool zero, const int* tune, long long& k) {
   const int nsweep = tune[11];
@@ -1563,10 +1570,7 @@ cudaError_t gs7_f32(cudaStream_t st, const MLevel& F, float* x, float* r, int fi
   } else if (zero) {
     e = cudaMemsetAsync(x, 0, F.g.n() * sizeof(float), st);
   }
-  const bool single = tune[5] == 2 ? (F.g.nx & 1) && (F.g.ny & 1)
-                                   : tune[5] == 0 && fint >= kSinglePassMin &&
-                                         gs7_rb_suits<float>(F.g.nx, F.g.ny, F.g.n(), tune[12]);
-  if (single) {
+  if (gs7_f32_single(F.g, tune)) {
     Gs7Rb<float> a = rb_f32(F, d32, tune);
     float *xin = x, *xout = xs;
     for (; sw < nsweep && e == cudaSuccess; sw++) {
@@ -2203,6 +2207,8 @@ int mixed_newton_inner(pmgb_solver* s, double errtol_s) {
   int it = 0;
   return refine(s, 1, F.cp, F.rhs, F.xt, errtol_s, 1000, 1, &it);
 }
+
+int mixed_fine_single(const pmgb_solver* s) { return gs7_f32_single(s->g, s->tune); }
 
 // One FP32 fine-level half-sweep for kernel timing; 5 FP32 arrays read and
 // x read/written: 12 B per point per half-sweep.

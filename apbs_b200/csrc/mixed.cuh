@@ -18,6 +18,8 @@ void set_error(const char* fmt, ...);
 int mixed_time_gs7(pmgb_solver* s, int parity, double* bytes);
 int mixed_prepare_sweep(pmgb_solver* s);
 int mixed_time_gs7_sweep(pmgb_solver* s, double* bytes);
+// Whether the fine level's FP32 sweeps take a single pass (else one per colour).
+int mixed_fine_single(const pmgb_solver* s);
 int mixed_time_tail(pmgb_solver* s, double* bytes);
 // FP64 path, LPBE: exact-to-round-off solve of the FP64 coarsest level
 // (FP64 refinement over FP32 V-cycles of extra Galerkin levels).

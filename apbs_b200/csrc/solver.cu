@@ -1629,6 +1629,15 @@ extern "C" int pmgb_solve_molecule(const pmgb_params* params, int precision, int
   return ok;
 }
 
+extern "C" int pmgb_fine_smoother(const pmgb_solver* s) {
+  if (!s) return -1;
+  if (s->precision == PMGB_MIXED)
+    return mixed_fine_single(s) ? PMGB_K_GS7_SWEEP_FP32 : PMGB_K_GS7_FP32;
+  return s->tune[PMGB_TUNE_GS7_COLOUR_PASSES] == 1 || !gs7_sweep_supported(s->g)
+             ? PMGB_K_GS7_FP64
+             : PMGB_K_GS7_SWEEP_FP64;
+}
+
 extern "C" int pmgb_time_kernel(pmgb_solver* s, int which, int reps, double* ms,
                                 double* bytes) {
   if (!s || !s->built || reps < 1) {

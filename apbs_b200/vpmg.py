@@ -114,6 +114,8 @@ def lib():
                                           ctypes.POINTER(PmgbStats)]
         L.pmgb_time_kernel.argtypes = [vp, ctypes.c_int, ctypes.c_int, dp, dp]
         L.pmgb_time_kernel.restype = ctypes.c_int
+        L.pmgb_fine_smoother.argtypes = [vp]
+        L.pmgb_fine_smoother.restype = ctypes.c_int
         L.pmgb_batch_solve.argtypes = [ctypes.POINTER(vp), ctypes.c_int, vp]
         L.pmgb_batch_solve.restype = ctypes.c_int
         L.pmgb_solver_set_tuning.argtypes = [vp, ctypes.c_int, ctypes.c_int]
@@ -302,6 +304,10 @@ class Vpmg:
 
     def get_tuning(self, key: int) -> int:
         return int(lib().pmgb_solver_get_tuning(self._h, key))
+
+    def fine_smoother(self) -> int:
+        """The K_* kernel that most of this calculation's fine-level sweeps run in."""
+        return int(lib().pmgb_fine_smoother(self._h))
 
     def time_kernel(self, which: int, reps: int = 20):
         """Mean device ms per launch and algorithmic bytes per launch."""

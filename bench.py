@@ -485,12 +485,10 @@ def main():
         # the fine smoother the tuned calculation runs: FP32 single-pass
         # sweeps or one launch per colour
         ksolver = solvers["mixed"]
-        if ksolver.get_tuning(vpmg.TUNE_GS7_COLOUR_PASSES) == 2:
-            kern, kname = vpmg.K_GS7_SWEEP_FP32, "k_gs7_rb<float>"
-        else:
-            kern, kname = vpmg.K_GS7_FP32, "k_gs7_f32"
+        kern = ksolver.fine_smoother()
+        kname = {vpmg.K_GS7_SWEEP_FP32: "k_gs7_rb<float>", vpmg.K_GS7_FP32: "k_gs7_f32"}[kern]
     else:
-        kern, kname, ksolver = vpmg.K_GS27_WAVE, "k_gs27_wave", solvers["fp64"]
+        kern, kname, ksolver = vpmg.K_GS27_WAVE, "k_gs27_mail", solvers["fp64"]
     ms, nbytes = ksolver.time_kernel(kern, 10)
     achieved = nbytes / (ms * 1e-3) / 1e9
     traffic = None

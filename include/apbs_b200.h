@@ -295,6 +295,10 @@ int pmgb_get_tuning(int key);
 int pmgb_solver_set_tuning(pmgb_solver *s, int key, int value);
 int pmgb_solver_get_tuning(pmgb_solver *s, int key);
 
+/* The kernel (PMGB_K_*) that most of this calculation's fine-level sweeps run
+ * in, by its grid and tunables: single-pass sweeps or one launch per colour. */
+int pmgb_fine_smoother(const pmgb_solver *s);
+
 /* Launch one kernel `reps` times back to back on the solver's stream (after
  * a solve, on its state) and report the mean device time per launch (CUDA
  * events) and the algorithmic bytes one launch must move. */
