@@ -51,7 +51,7 @@ CANDIDATES = {
         TUNE_TAIL_MAX_POINTS: [20000, 70000, 5000],
         TUNE_MIXED_FINE_SWEEPS: [2, 1, 3, 4],
         TUNE_MIXED_COARSE_SWEEPS: [2, 1, 3],
-        TUNE_GS7_COLOUR_PASSES: [0, 1, 2],
+        TUNE_GS7_COLOUR_PASSES: [0, 2],
         TUNE_GS7_SWEEP_SHAPE: [0x12, 0x21, 0x11],
         TUNE_GS7_SWEEP_KCHUNK: [0, 6, 8],
         TUNE_GS27_CLUSTER_MID: [0, 4, 16],

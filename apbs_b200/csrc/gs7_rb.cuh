@@ -237,19 +237,6 @@ inline cudaError_t launch_gs7_rb_nt(cudaStream_t st, const Gs7Rb<T>& a, int c1, 
 
 // shape: bits 0-3 threads per CTA (0: 256, 1: 512, 2: 1024), bits 4-7 pair
 // slots per thread (1-4, 0: 2); a CTA's widened range is threads x slots pairs
-inline int gs7_rb_range(int shape) {
-  const int nt = shape & 15, q = ((shape >> 4) & 15) ? ((shape >> 4) & 15) : 2;
-  return (nt == 1 ? 512 : nt == 2 ? 1024 : 256) * q;
-}
-
-// whether the kernel takes a grid in that shape with at least half of the widened
-// range its own
-template <typename T>
-inline bool gs7_rb_suits(int nx, int ny, size_t n, int shape) {
-  return (nx & 1) && (ny & 1) && n * sizeof(T) < 2147483647u &&
-         ((shape >> 4) & 15) <= 4 && 2 * (nx + 3) <= gs7_rb_range(shape);
-}
-
 template <typename T>
 inline cudaError_t launch_gs7_rb(cudaStream_t st, const Gs7Rb<T>& a, int c1, int shape) {
   const int nt = shape & 15, q = ((shape >> 4) & 15) ? ((shape >> 4) & 15) : 2;

@@ -1534,20 +1534,16 @@ Gs7Rb<float> rb_f32(const MLevel& F, const float* d32, const int* tune) {
 
 // The fine-level FP32 smoothing: tune[11] red-black sweeps, from x = 0 (zero) or
 // from x, then (r given) the residual.  Memory bounds a colour pass, the L2's up to
-// 129^3 and HBM above, so the first pass from zero only writes, the diagonal is one
-// array (oC + cc, as the single-pass sweep has it), and above kSinglePassMin points
-// (tune[5] == 0), or for tune[5] == 2, the other sweeps take a single pass out of
-// place (x -> xs -> x ...; after an odd count xs is copied back): two colour passes
-// 21.6 us and a single pass 22.7 at 129^3, 41.5 and 36.9 at 161^3, 118 and 89 at
-// 225^3.  An LPBE solve of 225^3 11.8 -> 10.6 ms and of 65^3 1.30 -> 1.22, the same
-// bits.  k counts the kernels launched.
-constexpr size_t kSinglePassMin = 3000000;
-
+// 129^3 and HBM above, so the first pass from zero only writes and the diagonal is
+// one array (oC + cc, as the single-pass sweep has it); an LPBE solve of 65^3 1.30 ->
+// 1.22 ms, the same bits.  Every sweep is two colour passes; for tune[5] == 2 those
+// after one from zero take a single pass out of place (x -> xs -> x ...; after an odd
+// count xs is copied back).  Alone the single pass is the faster one on large grids
+// (161^3 36.9 us against 41.5), in a solve it is not: an LPBE solve of 161^3 4.24 ms
+// against 4.11 in colours, 193^3 6.43 and 6.43, 225^3 10.77 and 10.85, 257^3 15.8 and
+// 15.5.  k counts the kernels launched.
 bool gs7_f32_single(Grid g, const int* tune) {
-  const size_t fint = (size_t)(g.nx - 2) * (g.ny - 2) * (g.nz - 2);
-  return tune[5] == 2 ? (g.nx & 1) && (g.ny & 1)
-                      : tune[5] == 0 && fint >= kSinglePassMin &&
-                            gs7_rb_suits<float>(g.nx, g.ny, g.n(), tune[12]);
+  return tune[5] == 2 && (g.nx & 1) && (g.ny & 1);
 }
 
 cudaError_t gs7_f32(cudaStream_t st, const MLevel& F, float* x, float* r, int first_parity,

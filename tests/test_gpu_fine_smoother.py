@@ -1,6 +1,5 @@
 """pmgb_fine_smoother names the kernel the fine sweeps run in (the benchmark times
-it): the mixed path's rule on points and the tunables' overrides, checked by the
-launches of a solve -- a single-pass sweep is one launch instead of two."""
+it) by the tunable, checked by the launches of a solve -- a single-pass sweep is one launch instead of two."""
 import pytest
 
 from apbs_b200 import synth
@@ -10,8 +9,8 @@ from apbs_b200.vpmg import (FP64, K_GS7_FP32, K_GS7_FP64, K_GS7_SWEEP_FP32, K_GS
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("dime,default", [(129, K_GS7_FP32), (161, K_GS7_SWEEP_FP32)])
-def test_mixed_fine_smoother_by_size_and_tunable(dime, default):
+@pytest.mark.parametrize("dime", [65, 161])
+def test_mixed_fine_smoother_by_tunable(dime):
     m = synth.cluster(60, 5.0, seed=2, net_charge=1.0)
     p = synth.mg_manual(dime, 30.0 / (dime - 1), m.center())
     per_cycle = {}
@@ -23,12 +22,12 @@ def test_mixed_fine_smoother_by_size_and_tunable(dime, default):
             lib().pmgb_launch_count(1)
             c.solve()
             per_cycle[value] = (lib().pmgb_launch_count(0) - 10.0) / c.stats()["vcycles"]
-            want = {0: default, 1: K_GS7_FP32, 2: K_GS7_SWEEP_FP32}[value]
+            want = {0: K_GS7_FP32, 1: K_GS7_FP32, 2: K_GS7_SWEEP_FP32}[value]
             assert c.fine_smoother() == want
     # two sweeps down (the first from zero, in colours either way) and two up: three
     # launches fewer per V-cycle, the solve's other launches aside
     assert per_cycle[1] - per_cycle[2] > 2.0
-    assert per_cycle[0] == per_cycle[2 if default == K_GS7_SWEEP_FP32 else 1]
+    assert per_cycle[0] == per_cycle[1]
 
 
 def test_fp64_fine_smoother():
