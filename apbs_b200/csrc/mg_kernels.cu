@@ -955,8 +955,8 @@ int launch_gs27_planes(cudaStream_t s, Grid g, Op op, const double* cc, const do
 //    for a pass that needs no order.
 // Measured (two sweeps and the residual; in brackets the kernels before, whole
 // planes in shared memory and a global mailbox, at 113^3 step counters):
-// 17^3 40 us (66), 33^3 68 (126), 49^3 98 (203), 65^3 135 (289), 81^3 215 (455),
-// 97^3 286 (744), 113^3 387 (1244).  One group of threads for all rows of a
+// 17^3 39 us (66), 33^3 68 (126), 49^3 98 (203), 65^3 135 (289), 81^3 215 (455),
+// 97^3 284 (744), 113^3 388 (1244).  One group of threads for all rows of a
 // half-sweep: 81^3 300, 49^3 150.
 //
 // Why a neighbour stays within wlag rows: half-sweep q of the lower plane can
@@ -981,8 +981,8 @@ constexpr int kPackPairs = 14;      // pairs of doubles per point of k_gs27_pack
 __host__ __device__ constexpr int mail_width(int hp) { return (hp + 31) / 32 * 32; }
 // Per row width: stages of packed coefficients per half-sweep, and rows between
 // successive half-sweeps at most -- the more, the less a plane's progress hangs
-// on its neighbours' (81^3: 294 us at 6 rows, 242 at 8; 49^3: 140, 113, 100 at
-// 12), as many as shared memory holds.
+// on its neighbours' (in the kernel's first form with two groups 81^3 took 294 us at
+// 6 rows and 242 at 8; 49^3 140, 113, and 100 at 12), as many as shared memory holds.
 __host__ __device__ constexpr int mail_stages(int hp) { return hp <= 40 ? 3 : 2; }
 __host__ __device__ constexpr int mail_lag(int hp) {
   return hp <= 32 ? 14 : (hp <= 40 ? 11 : (hp <= 48 ? 10 : 8));
@@ -1190,7 +1190,7 @@ __global__ void __launch_bounds__(2 * kMailHalfMax * mail_width(HP) + kMailHelpe
   asm volatile("cp.async.wait_all;" ::: "memory");
   cl.sync();  // every inbox of the cluster is clear before anyone writes one
   const unsigned tag = tag_sh;
-  const unsigned itag0 = tag * 64u + 1u;  // inbox tag of lap 0 (at most 113 / 7 laps)
+  const unsigned itag0 = tag * 64u + 1u;  // inbox tag of lap 0, others within the launch
   volatile int* verr = err;
   // a wait's bound: false once it ran out, here or elsewhere
   auto keep_waiting = [&](unsigned long long& t0) -> bool {

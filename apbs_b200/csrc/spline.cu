@@ -453,11 +453,12 @@ __device__ __forceinline__ void force_sum(double v[3], double (*sh)[3]) {
 }
 
 // One CTA per atom, its threads striding over the grid points of each sum.
-// What bounds it is the FP64 arithmetic of the points near the surface (six
-// square roots and divisions each); with one thread per atom the kernel ran
-// for as long as one thread took over all its atom's points (13.8 ms for 700
-// atoms at 0.6 A, 0.15 ms now).  The sums are the reference's terms in
-// another order.
+// What bounds it is the latency of the FP64 chains of the points near the surface
+// (six square roots and divisions each), with 12 warps of 144 registers to an SM:
+// FP64 pipe 18 % busy, memory under 4 %.
+// With one thread per atom the kernel ran for as long as one thread took over
+// all its atom's points (13.8 ms for 700 atoms at 0.6 A, 0.15 ms now).  The sums
+// are the reference's terms in another order.
 __global__ void __launch_bounds__(kForceThreads) k_forces(ForceArgs A) {
   __shared__ double sh[kForceThreads / 32][3];
   const int a = blockIdx.x;
