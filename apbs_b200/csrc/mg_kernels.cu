@@ -1594,6 +1594,7 @@ static MailPlan mail_plan(Grid g, int nhalf) {
 }
 
 int wave_mail_fit(Grid g) { return mail_plan(g, kMailHalfMax).kernel != nullptr; }
+int wave_mail_may_fit(Grid g) { return mail_kernel(g) && g.nz >= 4 && g.nz - 2 <= 148; }
 
 int launch_gs27_mail(cudaStream_t s, Grid g, const double* pack, const double* fc, double* x,
                      int x_zero, int nsweep, int first_parity, unsigned* counters, int* err,

@@ -79,7 +79,9 @@ int launch_gs27_wave(cudaStream_t s, Grid g, Op op, const double* cc, const doub
 // the device.  Returns 0 (nothing launched) where it does not fit.
 size_t mail_words(Grid g);
 size_t gs27_pack_doubles(Grid g);
+// wave_mail_may_fit: the same without asking the device (a B200's 148 SMs).
 int wave_mail_fit(Grid g);
+int wave_mail_may_fit(Grid g);
 // coef 0: only D = oC + cc and 1/D, for another cc on the packed operator
 void launch_gs27_pack(cudaStream_t s, Grid g, Op op, const double* cc, double* pack, int coef);
 int launch_gs27_mail(cudaStream_t s, Grid g, const double* pack, const double* fc, double* x,

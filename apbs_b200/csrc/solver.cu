@@ -526,11 +526,9 @@ extern "C" size_t pmgb_footprint(const pmgb_params* params, int precision, int n
   for (int l = 0; l < nlev; l++) d += (size_t)((l == 0 ? 4 : 14) + 7) * nl[l];
   size_t bytes = d * sizeof(double);
   bytes += 3 * n;  // the dielectric byte maps
-  // mailboxes and packed coefficients of the FP64 plane wavefront (an upper
-  // bound where the device has fewer SMs than the level planes)
+  // mailboxes and packed coefficients of the FP64 plane wavefront
   for (int l = 1; precision == PMGB_FP64 && l < nlev - 1; l++)
-    if (gx[l] <= 113) {
-      const Grid g{gx[l], gy[l], gz[l]};
+    if (const Grid g{gx[l], gy[l], gz[l]}; wave_mail_may_fit(g)) {
       bytes += mail_words(g) * sizeof(unsigned long long) + gs27_pack_doubles(g) * sizeof(double);
     }
   // FP32 hierarchy from level lo, plus Galerkin levels down to <= 512 unknowns
