@@ -58,10 +58,15 @@ struct OpF {
 
 }  // namespace
 
+// a divisor as quotient takes it (m 0: 1)
+struct Quot {
+  unsigned m, shift;
+};
+
 // one level of the FP32 hierarchy as seen by the tail kernel
 struct TLev {
   Grid g;
-  unsigned dx, dy;   // ceil(2^32 / (nx - 2)), ceil(2^32 / (ny - 2)): interior_at
+  Quot dx, dy;       // div_const of nx - 2 and ny - 2: interior_at
   const float* op[14];
   const float* cc;
   float* w0;
@@ -782,21 +787,22 @@ __device__ __forceinline__ float nb27t(const TLev& L, const float* x, size_t id)
   return nb27(o, L.g, x, id);
 }
 
-// q / d for 0 <= q < 2^31 by multiplication with c = div_const(d) = ceil(2^32 / d)
-// (0: d = 1): q c / 2^32 is q / d plus less than 1/2, so its whole part is the
-// quotient or one more (tests/test_long_axes.py).
-inline unsigned div_const(int d) {
-  return d > 1 ? (unsigned)((0x100000000ull + d - 1) / d) : 0u;
+// q / d for 0 <= q < 2^31 (T. Granlund, P. Montgomery, PLDI 1994): with l =
+// ceil(log2 d) and m = ceil(2^(31 + l) / d) < 2^32, q m / 2^(31 + l) exceeds q / d by
+// less than 1 / d, as q (m d - 2^(31 + l)) < 2^31 2^l (tests/test_long_axes.py).
+inline Quot div_const(int d) {
+  int l = 0;
+  while ((1ll << l) < d) l++;
+  if (l == 0) return Quot{0u, 0u};
+  return Quot{(unsigned)(((1ull << (31 + l)) + d - 1) / d), (unsigned)(l - 1)};
 }
-__device__ __forceinline__ int quotient(int q, int d, unsigned c) {
-  if (!c) return q;
-  const unsigned t = __umulhi((unsigned)q, c);
-  return (int)(t - (t * (unsigned)d > (unsigned)q ? 1u : 0u));
+__device__ __forceinline__ int quotient(int q, Quot c) {
+  return c.m ? (int)(__umulhi((unsigned)q, c.m) >> c.shift) : q;
 }
 // Interior point q of a level as a flat index.
-__device__ __forceinline__ int interior_at(Grid g, unsigned dx, unsigned dy, int q) {
+__device__ __forceinline__ int interior_at(Grid g, Quot dx, Quot dy, int q) {
   const int ex = g.nx - 2, ey = g.ny - 2;
-  const int t = quotient(q, ex, dx), k = quotient(t, ey, dy);
+  const int t = quotient(q, dx), k = quotient(t, dy);
   return ((k + 1) * g.ny + t - k * ey + 1) * g.nx + q - t * ex + 1;
 }
 
@@ -916,7 +922,7 @@ __device__ void tail_smooth(const TLev& L, int reverse, TailTid tid, int nsweep)
 template <int CLUSTER>
 __device__ void tail_cheb(const TLev& L, TailTid tid, int K, int first) {
   const Grid g = L.g;
-  const unsigned dx = L.dx, dy = L.dy;
+  const Quot dx = L.dx, dy = L.dy;
   OpF o;
 #pragma unroll
   for (int c = 0; c < 14; c++) o.c[c] = L.op[c];
@@ -991,7 +997,7 @@ template <int CLUSTER>
 __device__ void tail_damp(const TLev& L, TailTid tid, double* sh, double* slots,
                           int& phase, double& num, double& den) {
   const Grid g = L.g;
-  const unsigned dx = L.dx, dy = L.dy;
+  const Quot dx = L.dx, dy = L.dy;
   OpF o;
 #pragma unroll
   for (int c = 0; c < 14; c++) o.c[c] = L.op[c];
@@ -1016,7 +1022,7 @@ __device__ void tail_damp(const TLev& L, TailTid tid, double* sh, double* slots,
 }
 
 // xf += xdamp * (trilinear interpolation of xc) on the interior of gf
-__device__ void tail_interp(Grid gc, const float* xc, Grid gf, unsigned dx, unsigned dy, float* xf,
+__device__ void tail_interp(Grid gc, const float* xc, Grid gf, Quot dx, Quot dy, float* xf,
                             float xdamp, TailTid tid) {
   const int ex = gf.nx - 2, ey = gf.ny - 2, nint = ex * ey * (gf.nz - 2);
   struct Corrected {
@@ -1026,7 +1032,7 @@ __device__ void tail_interp(Grid gc, const float* xc, Grid gf, unsigned dx, unsi
   for_points<2>(
       nint, tid, [](int q) { return q; },
       [&](int q) {
-        const int t = quotient(q, ex, dx), k = quotient(t, ey, dy) + 1;
+        const int t = quotient(q, dx), k = quotient(t, dy) + 1;
         const int i = q - t * ex + 1, j = t - (k - 1) * ey + 1;
         const int ii = i >> 1, jj = j >> 1, kk = k >> 1;
         const int oi = i & 1, oj = j & 1, ok = k & 1;
@@ -1076,7 +1082,7 @@ __device__ void tail_cycle(const TailArgs& A, bool rhs_given, TailTid tid, doubl
       if (A.cheb > 0) tail_cheb<CLUSTER>(L, tid, A.cheb, cheb0 ? 1 : 0);
       else tail_smooth<CLUSTER>(L, 0, tid, A.nsweep);
       const Grid g = L.g;
-      const unsigned dx = L.dx, dy = L.dy;
+      const Quot dx = L.dx, dy = L.dy;
       const int nint = (g.nx - 2) * (g.ny - 2) * (g.nz - 2);
       OpF o;
 #pragma unroll
@@ -1284,7 +1290,7 @@ __global__ void __launch_bounds__(512) k_coarse_exact(ExactArgs E) {
 struct BatchItem {
   TailArgs T;             // FP32 levels 1 .. coarsest (T.first = 1)
   Grid g;                 // fine grid
-  unsigned dx, dy, dh;    // div_const of nx - 2, ny - 2 and the points of a colour in a row
+  Quot dx, dy, dh;        // div_const of nx - 2, ny - 2 and the points of a colour in a row
   const double* op[4];    // FP64 fine operator: oC oE oN uC
   const double* cc;
   const double* fc;
@@ -1305,7 +1311,7 @@ struct BatchItem {
 // x = 0 (zero: the first colour of the first sweep) the neighbours are not read,
 // and the other colour is set to 0
 template <int CLUSTER>
-__device__ void batch_gs7(const BatchItem& B, unsigned dh, unsigned dy, int parity, bool zero,
+__device__ void batch_gs7(const BatchItem& B, Quot dh, Quot dy, int parity, bool zero,
                           TailTid tid) {
   const Grid g = B.g;
   const int nx = g.nx, ny = g.ny, nz = g.nz;
@@ -1318,7 +1324,7 @@ __device__ void batch_gs7(const BatchItem& B, unsigned dh, unsigned dy, int pari
   for_points<4>(
       nslots, tid,
       [&](int q) {
-        const int t = quotient(q, hr, dh), k = quotient(t, ey, dy) + 1;
+        const int t = quotient(q, dh), k = quotient(t, dy) + 1;
         const int m = q - t * hr, j = t - (k - 1) * ey + 1;
         const int off = ((1 + j + k) & 1) != parity;
         const int i = 1 + off + 2 * m;
@@ -1360,7 +1366,7 @@ __global__ void __launch_bounds__(512) k_batch_solve(const BatchItem* __restrict
   const int ex = nx - 2, ey = ny - 2, nint = ex * ey * (g.nz - 2);
   const int n = (int)g.n();
   const int sy = nx, sz = nx * ny;
-  const unsigned dx = B.dx, dy = B.dy;
+  const Quot dx = B.dx, dy = B.dy;
   auto interior = [&](int q) { return interior_at(g, dx, dy, q); };
 
   // x = 0; ||f||_1 (Vxnrm1 on the interior)

@@ -13,11 +13,12 @@ from apbs_b200.vpmg import (FP64, MIXED, TUNE_GS7_COLOUR_PASSES, TUNE_TAIL_MAX_P
 
 
 def quotient(q, d):
-    c = (2**32 + d - 1) // d if d > 1 else 0
-    if not c:
+    bits = (d - 1).bit_length()
+    if bits == 0:
         return q
-    t = (q * c) >> 32
-    return t - ((t * d) % 2**32 > q)
+    m = (2**(31 + bits) + d - 1) // d
+    assert m < 2**32
+    return ((q * m) >> 32) >> (bits - 1)
 
 
 def test_quotient_is_exact_below_two_to_the_31():
